@@ -49,7 +49,7 @@ void Workspace::attach_arena(Arena* a) {
   DevBuf* bufs[] = {&model, &in, &ids, &dists, &xs, &ps, &psf, &pid, &keys0, &keys1, &vals0, &vals1, &hist,
                     &scan_tmp, &flags, &pos, &ckeys, &coff, &dstart, &list0, &list1, &small,
                     &eps_partial, &eps_sample, &perm, &minmax_part, &qradius, &chunk_list, &patch_rows, &defer_list,
-                    &fps, &fpid, &fdstart, &qorder, &rowsum};
+                    &fps, &fpid, &fdstart, &qorder, &rowsum, &tree_box, &tree_split};
   for (DevBuf* b : bufs) {
     b->arena = a;
     b->p = nullptr;
@@ -108,7 +108,7 @@ void Workspace::release_all() {
   DevBuf* bufs[] = {&model, &in, &ids, &dists, &xs, &ps, &psf, &pid, &keys0, &keys1, &vals0, &vals1, &hist,
                     &scan_tmp, &flags, &pos, &ckeys, &coff, &dstart, &list0, &list1, &small,
                     &eps_partial, &eps_sample, &perm, &minmax_part, &qradius, &chunk_list, &patch_rows, &defer_list,
-                    &fps, &fpid, &fdstart, &qorder, &rowsum};
+                    &fps, &fpid, &fdstart, &qorder, &rowsum, &tree_box, &tree_split};
   for (DevBuf* b : bufs) b->release();
   if (stream) cudaStreamDestroy(stream);
   stream = nullptr;
@@ -276,6 +276,7 @@ struct SmallDev {  // layout of Workspace::small
   uint32_t mlp_err;  // the tensor-core radius MLP timed out
   uint32_t chunk_fill[MAX_ROW_CHUNKS];  // streamed rows: queries placed per id block
   uint32_t patch_count;                 // streamed rows: first-pass failures
+  uint32_t tree_fail[2];                // tree search: failures of its first two passes
   unsigned long long defer_total;       // all queries handed over by the tile search in this join
 };
 
@@ -337,8 +338,9 @@ static void build_grid(Workspace& w, const JoinConfig& cfg, uint64_t n, uint32_t
   uint32_t* coff = (uint32_t*)w.coff.get((n + 1) * 4);
   SmallDev* sm = (SmallDev*)w.small.p;
   launch_compact_cells(skeys, n, flags, pos, sc.scan_tmp, ckeys, coff, &sm->C, s);
-  T* ps = (T*)w.ps.get(n * d * sizeof(T));
-  float* psf = sizeof(T) == 8 ? (float*)w.psf.get(n * d * sizeof(float)) : nullptr;
+  // (the box tree keeps its columns in the same buffers, at its own stride)
+  T* ps = (T*)w.ps.get(tree_stride(n) * d * sizeof(T));
+  float* psf = sizeof(T) == 8 ? (float*)w.psf.get(tree_stride(n) * d * sizeof(float)) : nullptr;
   uint32_t* pid = (uint32_t*)w.pid.get(n * 4);
   dev_copy(w, pid, sids, n * 4, s);
   launch_gather_sorted<T>(xs, n, d, sids, ps, psf, s);
@@ -605,6 +607,7 @@ template <typename T>
 struct Prepared {
   DeviceGrid<T> grid;
   T* xs = nullptr;
+  const T* minmax = nullptr;  // device: extremes of every column
   T eps0 = 0;
   int bucket = -1;
   double avg = 0.0;
@@ -704,6 +707,7 @@ static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T
   P->bucket = bucket;
   P->avg = head.avg[0];
   P->xs = xs;
+  P->minmax = d_minmax;
   if (st) {
     st->eps0 = (double)eps0;
     st->eps_bucket = bucket;
@@ -838,6 +842,102 @@ static bool run_graph_passes(Workspace& w, SearchLaunch<T> a, LoopCtl& c, LoopCt
   return true;
 }
 
+// Joins searched through the box tree.  Not those whose rows stream out in
+// blocks of ids during the first pass, nor those with a cap on the passes of
+// the radius schedule, which counts the schedule's own passes, nor double data
+// that the float screen cannot hold (or is told not to: the ring search then
+// takes every distance in double).  From four dimensions on the ring of cells
+// visits several times the points the tree does and most first passes fail
+// (10 M x 6-D: 3150 candidates per query in 10 passes against 2050 in 3).
+template <typename T>
+static bool tree_applies(const JoinConfig& cfg, uint32_t d, double max_abs, bool will_stream) {
+  if (!cfg.tree_search || will_stream || cfg.max_iterations > 0) return false;
+  if (sizeof(T) == 8 && (!cfg.float_prefilter || !(4.0 * std::sqrt((double)d) * max_abs < 1e18))) return false;
+  return cfg.tree_search == 2 || d >= 4;
+}
+
+struct TreePasses {
+  int passes = 1;
+  uint64_t queries_run = 0;
+  double ms = 0.0;    // device time of the search kernels
+  double rmax = 0.0;  // largest radius grown or searched (0: none)
+};
+
+// Builds the tree over the grid's point buffers (the grid is not searched
+// afterwards) and runs the passes: each reads its query count on the device,
+// so nothing waits for the host in between.
+template <typename T>
+static TreePasses run_tree(Workspace& w, const Prepared<T>& P, uint64_t n, uint32_t d,
+                           uint32_t di, uint32_t K, T* qrad, int32_t* d_ids, T* d_dists, double* rowsum, uint32_t* const* list, SmallDev* sm,
+                           cudaStream_t s) {
+  BoxTree<T> t;
+  tree_shape(n, d, t.count, t.offset, &t.levels, &t.nodes);
+  t.ld = tree_stride(n);
+  t.dims = std::min(d, TREE_DIMS);
+  t.ps = (T*)w.ps.get(t.ld * d * sizeof(T));
+  t.psf = sizeof(T) == 8 ? (float*)w.psf.get(t.ld * d * sizeof(float)) : nullptr;
+  t.id = (uint32_t*)w.pid.get(n * 4);
+  t.box = (float*)w.tree_box.get((size_t)2 * t.dims * t.nodes * 4);
+  TreeScratch sc;
+  sc.sort.keys[0] = (unsigned long long*)w.keys0.get(n * 8);
+  sc.sort.keys[1] = (unsigned long long*)w.keys1.get(n * 8);
+  sc.sort.vals[0] = (uint32_t*)w.vals0.get(n * 4);
+  sc.sort.vals[1] = (uint32_t*)w.vals1.get(n * 4);
+  sc.sort.hist_elems = radix_hist_elems(n);
+  sc.sort.hist = (uint32_t*)w.hist.get(sc.sort.hist_elems * 4);
+  sc.sort.scan_tmp_elems = scan_tmp_elems(std::max<size_t>(sc.sort.hist_elems, n + 1));
+  sc.sort.scan_tmp = (uint32_t*)w.scan_tmp.get(sc.sort.scan_tmp_elems * 4);
+  sc.split = (float*)w.tree_split.get(tree_split_elems() * 4);
+  launch_tree_build<T>(P.xs, P.minmax, n, d, sc, t, s);
+  launch_zero_words(sm->tree_fail, sizeof(sm->tree_fail), s);
+  launch_zero_words(&sm->fr, sizeof(FailRadii), s);
+  for (int i = 0; i < 2; i++) launch_zero_words(list[i], (size_t)t.count[0] * 4, s);
+  TreeLaunch<T> a;
+  a.tree = t;
+  a.n = n;
+  a.d = d;
+  a.K = K;
+  a.indexed = di;
+  a.radius = P.eps0;
+  a.qradius = qrad;
+  a.out_ids = d_ids;
+  a.out_d = d_dists;
+  a.rowsum = rowsum;
+  a.fail_mask = list[0];
+  a.fail_count = &sm->tree_fail[0];
+  a.grow = (T*)w.qradius.get(n * sizeof(T));
+  a.rmax_bits = &sm->fr.rmax_bits;
+  a.cand_count = &sm->cand;
+  if (w.ev[4]) KNNSJ_CUDA(cudaEventRecord(w.ev[4], s));
+  launch_tree_search<T>(a, w.sm_count, s);
+  a.qmask = list[0];
+  a.nq_dev = &sm->tree_fail[0];
+  a.qradius = a.grow;
+  a.fail_mask = list[1];
+  a.fail_count = &sm->tree_fail[1];
+  launch_tree_search<T>(a, w.sm_count, s);
+  a.qmask = list[1];
+  a.nq_dev = &sm->tree_fail[1];
+  a.qradius = nullptr;
+  a.unbounded = 1;
+  launch_tree_search<T>(a, w.sm_count, s);
+  if (w.ev[5]) KNNSJ_CUDA(cudaEventRecord(w.ev[5], s));
+  TreePasses r;
+  uint32_t fail[2];
+  unsigned long long bits = 0;
+  read_small(w, fail, sm->tree_fail, sizeof(fail), s);
+  read_small(w, &bits, &sm->fr.rmax_bits, sizeof(bits), s);
+  r.passes = 1 + (fail[0] > 0) + (fail[1] > 0);
+  r.queries_run = n + fail[0] + fail[1];
+  r.rmax = decode_radius<T>(bits);
+  if (w.ev[4] && w.ev[5]) {
+    float ms = 0.f;
+    KNNSJ_CUDA(cudaEventElapsedTime(&ms, w.ev[4], w.ev[5]));
+    r.ms = ms;
+  }
+  return r;
+}
+
 template <typename T>
 void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_aos, uint64_t n, uint32_t d,
               uint32_t k, int32_t* d_ids, T* d_dists, knnsj_stats* st, cudaStream_t s, RowStream* rows,
@@ -861,20 +961,23 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
   SmallDev* sm = (SmallDev*)w.small.p;
   rec(1);
 
+  const bool will_stream = rows && rows->chunks >= 2 && n >= (uint64_t)rows->chunks;
+  const bool use_tree = tree_applies<T>(cfg, d, P.max_abs, will_stream);
   // 5. starting radii: eps0 for every query (plain), or one per query
   T* qrad = nullptr;
   double rmax = (double)P.eps0;
   if (cfg.radius_mode == KNNSJ_RADIUS_LEARNED) {
     qrad = (T*)w.qradius.get(n * sizeof(T));
     KNNSJ_CUDA(cudaMemsetAsync(&sm->mlp_err, 0, 4, s));
+    // (a box-tree search does not care how many cells a radius spans)
+    const double max_cells = use_tree ? 64.0 : learned_max_cells(di);
     launch_radius_assign<T>(P.grid, n, d, k, (float)cfg.beta, device_model(w, s), (double)P.eps0,
-                            (float)cfg.radius_offset, qrad, &sm->mlp_err, w.sm_count, s);
-    rmax = (double)P.eps0 * learned_max_cells(di);
+                            (float)cfg.radius_offset, max_cells, qrad, &sm->mlp_err, w.sm_count, s);
+    rmax = (double)P.eps0 * max_cells;
   }
   // 5b. the first pass's tile search (2-D / 3-D float data, all indexed)
   TileSetup<T> tile;
-  const bool will_stream = rows && rows->chunks >= 2 && n >= (uint64_t)rows->chunks;
-  if (cfg.tile_search && tile_search_applies(d, di, K, P.grid.dense, sizeof(T))) {
+  if (!use_tree && cfg.tile_search && tile_search_applies(d, di, K, P.grid.dense, sizeof(T))) {
     // per-query starting radii: query tiles over a grid of width eps0/4; a
     // uniform radius: one warp per query over a grid of width eps0/2
     // (measured best for each on the 25M-point sky-like set).  Streamed rows
@@ -930,7 +1033,7 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
   // until the graph stops.
   // (the caller waits for the copies and patches the late rows in:
   // finish_row_stream)
-  const bool streamed = rows && rows->chunks >= 2 && n >= (uint64_t)rows->chunks;
+  const bool streamed = will_stream;
   bool checksum_done = false;  // streamed rows: the checksum of the final table is launched
   if (streamed) {
     w.ensure_copy_stream();
@@ -1049,6 +1152,20 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
     rmax = c.rmax;
     rgrid = c.rgrid;
     rmax_seen = c.rmax_seen;
+  }
+
+  // 6b. the box tree: every query at its starting radius, the failures at a
+  // radius grown from what they found, and the rest without a radius
+  if (use_tree) {
+    TreePasses tp = run_tree<T>(w, P, n, d, di, K, qrad, d_ids, d_dists, rowsum, list, sm, s);
+    iter = tp.passes;
+    regrids = 1;  // the index was rebuilt once, as the tree
+    queries_run = tp.queries_run;
+    kernel_ms += tp.ms;
+    alg_bytes += (double)tp.passes * n * d * sizeof(T) + (double)queries_run * d * sizeof(T) +
+                 (double)n * K * (4.0 + sizeof(T));
+    if (tp.rmax > 0.0) rmax_seen = std::max(qrad ? rmax_seen : 0.0, tp.rmax);
+    nq = 0;
   }
 
   while (nq > 0) {
@@ -1193,7 +1310,7 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
   if (st) {
     st->iterations = iter;
     st->regrids = regrids;
-    st->eps_final = qrad ? rmax_seen : (double)r;
+    st->eps_final = qrad || use_tree ? rmax_seen : (double)r;
     st->candidates = cand;
     st->queries_run = queries_run;
     st->kernel_launches = g_launches;

@@ -216,10 +216,10 @@ static bool mlp_on_tensor_cores() {
 
 template <typename T>
 void launch_radius_assign(const DeviceGrid<T>& g, uint64_t n, uint32_t d, uint32_t k, float beta,
-                          const float* d_model, double eps0, float offset, T* qradius, uint32_t* d_err, int sm_count,
-                          cudaStream_t s) {
+                          const float* d_model, double eps0, float offset, double max_cells, T* qradius,
+                          uint32_t* d_err, int sm_count, cudaStream_t s) {
   const float log_lo = std::log(1.0f / 16.0f);
-  const float log_hi = (float)std::log(learned_max_cells(g.geom.di) * (1.0 - 1.0 / 4096.0));
+  const float log_hi = (float)std::log(max_cells * (1.0 - 1.0 / 4096.0));
   // the model predicts the 0.9 quantile of log(r_K / eps0); a failed first
   // pass costs a second scan at a larger radius, so starting 8% wider (in
   // radius) is cheaper overall (measured on 2-D, 3-D and 4-D joins, k 32-64)
@@ -255,9 +255,9 @@ void launch_mlp_predict(const float* d_model, const float* d_feat, uint64_t n, f
 }
 
 template void launch_radius_assign<float>(const DeviceGrid<float>&, uint64_t, uint32_t, uint32_t, float,
-                                          const float*, double, float, float*, uint32_t*, int, cudaStream_t);
+                                          const float*, double, float, double, float*, uint32_t*, int, cudaStream_t);
 template void launch_radius_assign<double>(const DeviceGrid<double>&, uint64_t, uint32_t, uint32_t, float,
-                                           const float*, double, float, double*, uint32_t*, int, cudaStream_t);
+                                           const float*, double, float, double, double*, uint32_t*, int, cudaStream_t);
 template void launch_radius_features<float>(const DeviceGrid<float>&, uint64_t, uint32_t, uint32_t, float, float*,
                                             cudaStream_t);
 template void launch_radius_features<double>(const DeviceGrid<double>&, uint64_t, uint32_t, uint32_t, float, float*,

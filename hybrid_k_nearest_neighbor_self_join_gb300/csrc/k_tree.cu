@@ -1,0 +1,365 @@
+// k_tree.cu -- build of the box tree the searches of tree_search.cuh walk.
+//
+// No counterpart in the reference, whose only index is the epsilon grid
+// (GPU.cu:3715-4067).  A grid of cells as wide as the radius needs 3^d cells
+// per query and one width for every density; the tree adapts to both: its
+// boxes hold 32 points each whatever the density, and a query visits only the
+// boxes its own radius reaches.
+//
+//   1. Quantiles of each key dimension from a strided sample (one block per
+//      dimension), so that the curve's cells hold similar numbers of points
+//      however the coordinates are distributed (far outliers, clumps).
+//   2. Hilbert-curve position of every point over those quantile
+//      coordinates, and a radix sort of (position, point).
+//   3. Blocks of 1024 consecutive points: five levels of splits at the
+//      median of the dimension of largest variance, in shared memory, make
+//      32 leaves of 32 points; the block writes its points, ids, leaf boxes
+//      and its own box.  On clustered 6-D and 8-D sets a query then reaches
+//      20-35 % fewer leaves than with leaves cut straight from the curve.
+//   4. The boxes of every 32 nodes, up to a level of at most 32 nodes (one
+//      block: a 32nd of the nodes per level).
+
+#include <algorithm>
+#include <cmath>
+
+#include "knnsj_internal.h"
+
+namespace knnsj {
+
+namespace {
+
+constexpr int SAMPLE = 4096;          // quantile sample per dimension
+constexpr int SPLIT_THREADS = 1024;
+constexpr int BLOCK_PTS = 1024;       // points of one refined block (32 leaves)
+constexpr int REFINE_THREADS = 512;
+constexpr uint32_t REFINE_DIMS = 16;  // dimensions considered by the median splits
+
+// Quantiles of dimension blockIdx.x: split[0] and split[TREE_BINS] are the
+// extremes of the whole column, the others sample quantiles.
+template <typename T>
+__global__ void __launch_bounds__(SPLIT_THREADS) tree_split_kernel(const T* __restrict__ xs, const T* __restrict__ mm,
+                                                                   uint64_t n, float* __restrict__ split) {
+  __shared__ float v[SAMPLE];
+  const uint32_t j = blockIdx.x;
+  const uint32_t m = (uint32_t)min((unsigned long long)n, (unsigned long long)SAMPLE);
+  uint32_t m2 = 1;
+  while (m2 < m) m2 <<= 1;
+  for (uint32_t i = threadIdx.x; i < m2; i += SPLIT_THREADS)
+    v[i] = i < m ? (float)xs[(uint64_t)j * n + (uint64_t)i * n / m] : __int_as_float(0x7f800000);
+  __syncthreads();
+  for (uint32_t size = 2; size <= m2; size <<= 1) {
+    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+      for (uint32_t i = threadIdx.x; i < (m2 >> 1); i += SPLIT_THREADS) {
+        const uint32_t lo = ((i & ~(stride - 1)) << 1) | (i & (stride - 1));
+        const float a = v[lo], b = v[lo + stride];
+        if ((b < a) == ((lo & size) == 0)) {
+          v[lo] = b;
+          v[lo + stride] = a;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (uint32_t b = threadIdx.x; b <= TREE_BINS; b += SPLIT_THREADS) {
+    float x;
+    if (b == 0)
+      x = (float)mm[2 * j];
+    else if (b == TREE_BINS)
+      x = (float)mm[2 * j + 1];
+    else
+      x = v[(uint64_t)b * m / TREE_BINS];
+    split[j * (TREE_BINS + 1) + b] = x;
+  }
+}
+
+// Hilbert-curve position over the quantile coordinates of the first hd
+// dimensions, `bits` bits each (J. Skilling, "Programming the Hilbert curve",
+// 2004: Gray-code transpose, then the bits interleaved from the top).
+template <typename T>
+__global__ void tree_key_kernel(const T* __restrict__ xs, uint64_t n, uint32_t hd, int bits,
+                                const float* __restrict__ split, unsigned long long* __restrict__ keys,
+                                uint32_t* __restrict__ vals) {
+  __shared__ float sp[TREE_KEY_DIMS * (TREE_BINS + 1)];
+  for (uint32_t i = threadIdx.x; i < hd * (TREE_BINS + 1); i += blockDim.x) sp[i] = split[i];
+  __syncthreads();
+  const float top = (float)(1u << bits);
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    uint32_t X[TREE_KEY_DIMS];
+#pragma unroll
+    for (uint32_t j = 0; j < TREE_KEY_DIMS; j++) {
+      X[j] = 0;
+      if (j < hd) {
+        const float v = (float)xs[(uint64_t)j * n + i];
+        const float* q = sp + j * (TREE_BINS + 1);
+        uint32_t lo = 0;  // last bin whose lower edge is <= v
+#pragma unroll
+        for (uint32_t step = TREE_BINS / 2; step > 0; step >>= 1)
+          if (q[lo + step] <= v) lo += step;
+        const float w = q[lo + 1] - q[lo];
+        float f = w > 0.0f ? (v - q[lo]) / w : 0.0f;
+        f = fminf(fmaxf(f, 0.0f), 0.999f);
+        X[j] = min((uint32_t)(((float)lo + f) * (top / (float)TREE_BINS)), (1u << bits) - 1u);
+      }
+    }
+    for (uint32_t m = 1u << (bits - 1); m > 1; m >>= 1) {
+      const uint32_t low = m - 1;
+#pragma unroll
+      for (uint32_t j = 0; j < TREE_KEY_DIMS; j++) {
+        if (j < hd) {
+          if (X[j] & m) {
+            X[0] ^= low;
+          } else {
+            const uint32_t t = (X[0] ^ X[j]) & low;
+            X[0] ^= t;
+            X[j] ^= t;
+          }
+        }
+      }
+    }
+    uint32_t last = 0;
+#pragma unroll
+    for (uint32_t j = 1; j < TREE_KEY_DIMS; j++)
+      if (j < hd) X[j] ^= X[j - 1];
+#pragma unroll
+    for (uint32_t j = 0; j < TREE_KEY_DIMS; j++)
+      if (j + 1 == hd) last = X[j];
+    uint32_t t = 0;
+    for (uint32_t m = 1u << (bits - 1); m > 1; m >>= 1)
+      if (last & m) t ^= m - 1;
+    unsigned long long code = 0;
+    for (int b = bits - 1; b >= 0; b--) {
+#pragma unroll
+      for (uint32_t j = 0; j < TREE_KEY_DIMS; j++)
+        if (j < hd) code = (code << 1) | (((X[j] ^ t) >> b) & 1u);
+    }
+    keys[i] = code;
+    vals[i] = (uint32_t)i;
+  }
+}
+
+// floats as unsigned integers of the same order
+__device__ __forceinline__ uint32_t float_order(float x) {
+  const uint32_t b = __float_as_uint(x);
+  return b & 0x80000000u ? ~b : b | 0x80000000u;
+}
+__device__ __forceinline__ float order_float(uint32_t o) {
+  return __uint_as_float(o & 0x80000000u ? o & 0x7fffffffu : ~o);
+}
+__device__ __forceinline__ float box_down(float x) { return x; }
+__device__ __forceinline__ float box_down(double x) { return __double2float_rd(x); }
+__device__ __forceinline__ float box_up(float x) { return x; }
+__device__ __forceinline__ float box_up(double x) { return __double2float_ru(x); }
+
+// One block of 1024 consecutive points of the curve order: median splits down
+// to 32 leaves, then its points, ids and boxes.  Dynamic shared memory: the
+// first rd coordinates of the points as floats.
+template <typename T>
+__global__ void __launch_bounds__(REFINE_THREADS) tree_refine_kernel(const T* __restrict__ xs, uint64_t n, uint32_t d,
+                                                                     uint32_t rd, const uint32_t* __restrict__ ids,
+                                                                     T* __restrict__ ps, float* __restrict__ psf,
+                                                                     uint32_t* __restrict__ tid, uint64_t ld,
+                                                                     float* __restrict__ box, uint32_t nodes,
+                                                                     uint32_t bd, uint32_t leaves, uint32_t off1) {
+  extern __shared__ float co[];  // [rd][BLOCK_PTS]
+  __shared__ unsigned long long key[BLOCK_PTS];
+  __shared__ float var[16][REFINE_DIMS];
+  __shared__ uint32_t seg_dim[16];
+  const int tidx = threadIdx.x, lane = tidx & 31, warp = tidx >> 5;
+  constexpr int WARPS = REFINE_THREADS / 32;
+  const uint64_t base = (uint64_t)blockIdx.x * BLOCK_PTS;
+  const uint32_t cnt = (uint32_t)min((unsigned long long)BLOCK_PTS, (unsigned long long)(n - base));
+  for (uint32_t l = 0; l < rd; l++)
+    for (uint32_t i = tidx; i < cnt; i += REFINE_THREADS) co[l * BLOCK_PTS + i] = (float)xs[(uint64_t)l * n + ids[base + i]];
+  for (uint32_t i = tidx; i < BLOCK_PTS; i += REFINE_THREADS) key[i] = i;
+  __syncthreads();
+  for (uint32_t S = BLOCK_PTS; S > 32; S >>= 1) {
+    // variance of each dimension over each segment's points (padding sits at
+    // the end of the order)
+    const uint32_t segs = BLOCK_PTS / S;
+    for (uint32_t w = warp; w < segs * rd; w += WARPS) {
+      const uint32_t sg = w / rd, l = w % rd;
+      float s1 = 0.0f, s2 = 0.0f, c0 = 0.0f;
+      uint32_t m = 0;
+      if (sg * S < cnt) {
+        c0 = co[l * BLOCK_PTS + (uint32_t)(key[sg * S] & 1023u)];
+        for (uint32_t i = sg * S + lane; i < (sg + 1) * S; i += 32) {
+          const uint32_t loc = (uint32_t)(key[i] & 1023u);
+          if (loc < cnt) {
+            const float x = co[l * BLOCK_PTS + loc] - c0;
+            s1 += x;
+            s2 += x * x;
+            m++;
+          }
+        }
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        s1 += __shfl_xor_sync(FULL, s1, off);
+        s2 += __shfl_xor_sync(FULL, s2, off);
+        m += __shfl_xor_sync(FULL, m, off);
+      }
+      if (lane == 0) var[sg][l] = m ? s2 - s1 * (s1 / (float)m) : 0.0f;
+    }
+    __syncthreads();
+    if ((uint32_t)tidx < segs) {
+      uint32_t b = 0;
+      for (uint32_t l = 1; l < rd; l++)
+        if (var[tidx][l] > var[tidx][b]) b = l;
+      seg_dim[tidx] = b;
+    }
+    __syncthreads();
+    for (uint32_t i = tidx; i < BLOCK_PTS; i += REFINE_THREADS) {
+      const uint32_t loc = (uint32_t)(key[i] & 1023u);
+      const uint32_t o = loc < cnt ? float_order(co[seg_dim[i / S] * BLOCK_PTS + loc]) : 0xffffffffu;
+      key[i] = ((unsigned long long)o << 10) | loc;
+    }
+    __syncthreads();
+    // bitonic sort of every segment (ascending); a warp's pairs span 64
+    // consecutive keys once the stride is at most 32
+    for (uint32_t size = 2; size <= S; size <<= 1) {
+      for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+        const uint32_t i = tidx;
+        const uint32_t lo = ((i & ~(stride - 1)) << 1) | (i & (stride - 1));
+        const unsigned long long a = key[lo], b = key[lo + stride];
+        if ((b < a) == (size == S || (lo & size) == 0)) {
+          key[lo] = b;
+          key[lo + stride] = a;
+        }
+        if (stride > 32)
+          __syncthreads();
+        else
+          __syncwarp();
+      }
+      __syncthreads();
+    }
+  }
+  // points, ids and leaf boxes: a warp takes a leaf at a time
+  uint32_t* lob = reinterpret_cast<uint32_t*>(key);  // [bd][32] after the order is read
+  uint32_t loc[2];
+  for (int h = 0; h < 2; h++) loc[h] = (uint32_t)(key[(warp + h * WARPS) * 32 + lane] & 1023u);
+  __syncthreads();
+  uint32_t* hib = lob + TREE_DIMS * 32;
+  for (int h = 0; h < 2; h++) {
+    const uint32_t leaf = warp + h * WARPS;
+    const uint64_t pos = base + leaf * 32 + lane;
+    const bool live = leaf * 32 + lane < cnt;
+    const uint32_t id = live ? ids[base + loc[h]] : 0u;
+    if (live) tid[pos] = id;
+    for (uint32_t l = 0; l < d; l++) {
+      const T v = live ? xs[(uint64_t)l * n + id] : (T)0;
+      if (live) {
+        ps[(uint64_t)l * ld + pos] = v;
+        if (psf) psf[(uint64_t)l * ld + pos] = (float)v;
+      }
+      if (l < bd) {
+        const uint32_t lo = __reduce_min_sync(FULL, live ? float_order(box_down(v)) : 0xffffffffu);
+        const uint32_t hi = __reduce_max_sync(FULL, live ? float_order(box_up(v)) : 0u);
+        if (lane == 0) {
+          lob[l * 32 + leaf] = lo;
+          hib[l * 32 + leaf] = hi;
+          const uint32_t node = blockIdx.x * 32 + leaf;
+          if (node < leaves) {
+            box[(uint64_t)(2 * l) * nodes + node] = order_float(lo);
+            box[(uint64_t)(2 * l + 1) * nodes + node] = order_float(hi);
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (off1 != 0xffffffffu)
+    for (uint32_t l = warp; l < bd; l += WARPS) {
+      const uint32_t lo = __reduce_min_sync(FULL, lob[l * 32 + lane]);
+      const uint32_t hi = __reduce_max_sync(FULL, hib[l * 32 + lane]);
+      if (lane == 0) {
+        box[(uint64_t)(2 * l) * nodes + off1 + blockIdx.x] = order_float(lo);
+        box[(uint64_t)(2 * l + 1) * nodes + off1 + blockIdx.x] = order_float(hi);
+      }
+    }
+}
+
+// The levels above level 1, one after the other (one block).
+struct TreeLevels {
+  int levels;
+  uint32_t count[TREE_MAX_LEVELS], offset[TREE_MAX_LEVELS];
+};
+__global__ void __launch_bounds__(1024) tree_upper_kernel(float* __restrict__ box, uint32_t nodes, uint32_t bd,
+                                                          const TreeLevels lv) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int h = 2; h < lv.levels; h++) {
+    for (uint32_t w = warp; w < lv.count[h] * bd; w += 32) {
+      const uint32_t l = w / lv.count[h], nd = w % lv.count[h];
+      const uint32_t ch = nd * 32 + lane;
+      const bool there = ch < lv.count[h - 1];
+      float* lo = box + (uint64_t)(2 * l) * nodes;
+      float* hi = lo + nodes;
+      const uint32_t a = __reduce_min_sync(FULL, there ? float_order(lo[lv.offset[h - 1] + ch]) : 0xffffffffu);
+      const uint32_t b = __reduce_max_sync(FULL, there ? float_order(hi[lv.offset[h - 1] + ch]) : 0u);
+      if (lane == 0) {
+        lo[lv.offset[h] + nd] = order_float(a);
+        hi[lv.offset[h] + nd] = order_float(b);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+}  // namespace
+
+void tree_shape(uint64_t n, uint32_t d, uint32_t* count, uint32_t* offset, int* levels, uint32_t* nodes) {
+  (void)d;
+  uint64_t c = (n + 31) / 32, at = 0;
+  int h = 0;
+  for (;; h++) {
+    count[h] = (uint32_t)c;
+    offset[h] = (uint32_t)at;
+    at += (c + 31) & ~31ull;
+    if (c <= 32) break;
+    c = (c + 31) / 32;
+  }
+  *levels = h + 1;
+  *nodes = (uint32_t)at;
+}
+
+template <typename T>
+void launch_tree_build(const T* xs, const T* minmax, uint64_t n, uint32_t d, TreeScratch& sc, const BoxTree<T>& t,
+                       cudaStream_t s) {
+  const uint32_t hd = std::min<uint32_t>(d, TREE_KEY_DIMS);
+  tree_split_kernel<T><<<hd, SPLIT_THREADS, 0, s>>>(xs, minmax, n, sc.split);
+  KNNSJ_CHECK_LAUNCH();
+  // bits per dimension: enough for cells of well under one point on average;
+  // the blocks of 1024 points are ordered inside by the median splits
+  int log2n = 1;
+  while (log2n < 31 && (1ull << log2n) < n) log2n++;
+  int bits = (log2n + 8 + (int)hd - 1) / (int)hd;
+  bits = std::max(2, std::min({bits, 16, (int)(60 / hd)}));
+  const unsigned blocks = (unsigned)std::min<uint64_t>((n + 255) / 256, 152ull * 32);
+  tree_key_kernel<T><<<blocks, 256, 0, s>>>(xs, n, hd, bits, sc.split, sc.sort.keys[0], sc.sort.vals[0]);
+  KNNSJ_CHECK_LAUNCH();
+  const int cur = radix_sort_pairs(sc.sort, n, bits * (int)hd, s);
+  const uint32_t rd = std::min<uint32_t>(d, REFINE_DIMS);
+  const size_t smem = (size_t)rd * BLOCK_PTS * 4;
+  KNNSJ_CUDA(cudaFuncSetAttribute(tree_refine_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  tree_refine_kernel<T><<<(unsigned)((n + BLOCK_PTS - 1) / BLOCK_PTS), REFINE_THREADS, smem, s>>>(
+      xs, n, d, rd, sc.sort.vals[cur], const_cast<T*>(t.ps), const_cast<float*>(t.psf), const_cast<uint32_t*>(t.id),
+      t.ld, const_cast<float*>(t.box), t.nodes, t.dims, t.count[0], t.levels > 1 ? t.offset[1] : 0xffffffffu);
+  KNNSJ_CHECK_LAUNCH();
+  if (t.levels > 2) {
+    TreeLevels lv;
+    lv.levels = t.levels;
+    for (int h = 0; h < TREE_MAX_LEVELS; h++) {
+      lv.count[h] = t.count[h];
+      lv.offset[h] = t.offset[h];
+    }
+    tree_upper_kernel<<<1, 1024, 0, s>>>(const_cast<float*>(t.box), t.nodes, t.dims, lv);
+    KNNSJ_CHECK_LAUNCH();
+  }
+}
+
+template void launch_tree_build<float>(const float*, const float*, uint64_t, uint32_t, TreeScratch&,
+                                       const BoxTree<float>&, cudaStream_t);
+template void launch_tree_build<double>(const double*, const double*, uint64_t, uint32_t, TreeScratch&,
+                                        const BoxTree<double>&, cudaStream_t);
+
+}  // namespace knnsj

@@ -33,6 +33,8 @@ struct JoinConfig {
   int search_buffer = 0;
   int tail_brute = 1;                      // a few queries whose radius outgrew the grid are finished by
                                            // an exact scan over all points (2: at any due rebuild; 0: off)
+  int tree_search = 1;                     // box-tree search (tree_search.cuh): 0 off, 1 where it applies,
+                                           // 2 for every dimension count
   int row_chunks = 32;                     // with direct_rows 0: rows streamed out of the device table
                                            // in this many blocks while the join runs (< 2: at the end)
   int tile_search = 1;                     // first pass of 2-D / 3-D float data over a finer grid: 0 off,

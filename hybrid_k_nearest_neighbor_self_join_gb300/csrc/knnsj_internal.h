@@ -255,6 +255,60 @@ struct RowStream {
   double total_distance = 0.0;
 };
 
+// ---- box tree (k_tree.cu, tree_search.cuh) ---------------------------------
+// The points in an order that keeps neighbours together, 32 to a leaf, and
+// the bounding boxes of the leaves and of every 32 nodes above them.
+constexpr int TREE_MAX_LEVELS = 6;   // 32^6 leaves
+constexpr uint32_t TREE_DIMS = 16;   // dimensions the boxes cover (the first ones: largest variance)
+template <typename T>
+struct BoxTree {
+  const T* ps = nullptr;         // columns in tree order, stride ld
+  const float* psf = nullptr;    // double data: the same rounded to float (the float screen)
+  const uint32_t* id = nullptr;  // original id of each tree position
+  const float* box = nullptr;    // [2 * dims][nodes]: lower and upper bound of each dimension
+  uint64_t ld = 0;
+  uint32_t dims = 0;             // min(d, TREE_DIMS)
+  uint32_t nodes = 0;
+  int levels = 0;                // level 0: the leaves; the last level has at most 32 nodes
+  uint32_t count[TREE_MAX_LEVELS] = {};
+  uint32_t offset[TREE_MAX_LEVELS] = {};
+};
+struct TreeScratch {
+  GridScratch sort;          // keys, vals, hist, scan_tmp
+  float* split = nullptr;    // tree_split_elems()
+};
+constexpr uint32_t TREE_KEY_DIMS = 8;    // dimensions of the space-filling curve
+constexpr uint32_t TREE_BINS = 256;      // quantile bins per dimension
+constexpr size_t tree_split_elems() { return (size_t)TREE_KEY_DIMS * (TREE_BINS + 1); }
+inline uint64_t tree_stride(uint64_t n) { return (n + 31) & ~31ull; }
+void tree_shape(uint64_t n, uint32_t d, uint32_t* count, uint32_t* offset, int* levels, uint32_t* nodes);
+// Builds the tree of the n points given as input-order columns xs (stride n)
+// into t's buffers (ps, psf, id, box; shape set).
+template <typename T>
+void launch_tree_build(const T* xs, const T* minmax, uint64_t n, uint32_t d, TreeScratch& sc, const BoxTree<T>& t,
+                       cudaStream_t s);
+template <typename T>
+struct TreeLaunch {
+  BoxTree<T> tree;
+  uint64_t n = 0;
+  uint32_t d = 0, K = 0, indexed = 1;
+  const uint32_t* qmask = nullptr;   // bit b of word L: tree position 32 L + b is a query (nullptr: all)
+  const uint32_t* nq_dev = nullptr;  // with qmask: how many there are
+  T radius = 0;
+  T* qradius = nullptr;              // per-query radii by original id
+  int unbounded = 0;
+  int32_t* out_ids = nullptr;
+  T* out_d = nullptr;
+  double* rowsum = nullptr;
+  uint32_t* fail_mask = nullptr;     // bits of the failed queries (cleared before the pass)
+  uint32_t* fail_count = nullptr;
+  T* grow = nullptr;                 // grown radii of the failures, by original id
+  unsigned long long* rmax_bits = nullptr;  // largest radius grown or (without radii) searched
+  unsigned long long* cand_count = nullptr;
+};
+template <typename T>
+void launch_tree_search(const TreeLaunch<T>& a, int sm_count, cudaStream_t s);
+
 // ---- per-device workspace --------------------------------------------------
 struct Workspace {
   DevBuf model;                          // radius model (learned starting radius)
@@ -268,6 +322,7 @@ struct Workspace {
   DevBuf defer_list;                     // queries the tile search hands to search_kernel
   DevBuf rowsum;                         // per-row verification sums (host-pointer calls)
   DevBuf fps, fpid, fdstart;             // tile search: the finer candidate grid (columns, ids, start table)
+  DevBuf tree_box, tree_split;           // box tree: node boxes, quantiles (points and ids in ps, psf, pid)
   DevBuf qorder;                         // tile search: cell-ordered positions in Morton order of their cells
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[8] = {};
@@ -313,8 +368,8 @@ void run_features(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* 
 double learned_max_cells(uint32_t di);
 template <typename T>
 void launch_radius_assign(const DeviceGrid<T>& g, uint64_t n, uint32_t d, uint32_t k, float beta,
-                          const float* d_model, double eps0, float offset, T* qradius, uint32_t* d_err, int sm_count,
-                          cudaStream_t s);
+                          const float* d_model, double eps0, float offset, double max_cells, T* qradius,
+                          uint32_t* d_err, int sm_count, cudaStream_t s);
 template <typename T>
 void launch_radius_features(const DeviceGrid<T>& g, uint64_t n, uint32_t d, uint32_t k, float beta, float* out,
                             cudaStream_t s);

@@ -88,7 +88,8 @@ typedef struct {
 typedef struct {
   uint32_t struct_size;
   int32_t iterations;        /* search passes run */
-  int32_t regrids;           /* grid rebuilds at a coarser cell width */
+  int32_t regrids;           /* index rebuilds after the eps0 grid: grids of a coarser
+                                cell width, or (once) the box tree */
   int32_t eps_bucket;        /* histogram bucket that chose eps0 (GPU.cu:3510) */
   double eps0;               /* initial epsilon (DTYPE widened to double) */
   double eps_final;          /* largest radius searched */
