@@ -647,7 +647,11 @@ static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T
   launch_zero_words(&sm->defer_total, sizeof(sm->defer_total), s);
   KNNSJ_CUDA(cudaMemcpyAsync(d_perm, perm.data(), d * 4, cudaMemcpyHostToDevice, s));
   T* xs = (T*)w.xs.get(n * d * sizeof(T));
-  launch_transpose_reorder<T>(d_aos, xs, n, d, d_perm, s, &sm->nonfinite);
+  // (double data: a float copy too, for the histogram's brackets; the buffer
+  // later holds the cell-ordered float columns)
+  float* xsf = sizeof(T) == 8 ? (float*)w.psf.get(tree_stride(n) * d * sizeof(float)) : nullptr;
+  launch_transpose_reorder<T>(d_aos, xs, xsf, n, d, d_perm, s, &sm->nonfinite);
+  if (!xsf) xsf = reinterpret_cast<float*>(xs);
   T* mm_part = (T*)w.minmax_part.get(1024 * 2 * d * sizeof(T) + 2 * d * sizeof(T));
   T* d_minmax = mm_part + 1024 * 2 * d;
   launch_minmax<T>(xs, n, d, d_minmax, mm_part, s);
@@ -679,12 +683,12 @@ static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T
   // buckets [0, 256) first; the rest only if the crossing lies beyond
   std::vector<uint32_t> hh(10000, 0);
   const uint32_t first_range = 256;
-  launch_eps_hist<T>(xs, n, d, es, 0, first_range, abs_err, s);
+  launch_eps_hist<T>(xs, xsf, n, d, es, head.avg[0], 0, first_range, abs_err, s);
   KNNSJ_CUDA(cudaMemcpyAsync(hh.data(), sm->hist, first_range * 4, cudaMemcpyDeviceToHost, s));
   KNNSJ_CUDA(cudaStreamSynchronize(s));
   EpsChoice ec = choose_eps(hh.data(), first_range, head.avg[0], n, k, cfg.beta);
   if (!ec.complete) {
-    launch_eps_hist<T>(xs, n, d, es, first_range, 10000, abs_err, s);
+    launch_eps_hist<T>(xs, xsf, n, d, es, head.avg[0], first_range, 10000, abs_err, s);
     KNNSJ_CUDA(cudaMemcpyAsync(hh.data(), sm->hist, 10000 * 4, cudaMemcpyDeviceToHost, s));
     KNNSJ_CUDA(cudaStreamSynchronize(s));
     ec = choose_eps(hh.data(), 10000, head.avg[0], n, k, cfg.beta);

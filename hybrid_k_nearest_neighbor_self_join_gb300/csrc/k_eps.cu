@@ -26,6 +26,8 @@
 // are computed exactly as the reference does.  The bucket is always the
 // reference's double-precision bucket.
 
+#include <cmath>
+
 #include "exact_sqrt.cuh"
 #include "knnsj_internal.h"
 
@@ -147,40 +149,65 @@ __device__ __forceinline__ uint32_t exact_bucket(double rd, double avg, double b
   return b < NBUCKETS ? b : NBUCKETS;
 }
 
-// Counts the buckets in [b_lo, b_hi) of sample blocks.  abs_err bounds the
-// float bracket's absolute distance error from rounding the coordinates to
-// float (0 for float data).
+// The constants of a histogram launch, from the mean distance the host has
+// read by then.  (Computed by every thread on the device, their double
+// divisions took 1/64-rate FP64 time in each of the 8000 blocks: 222 us for
+// 100 000 points, whose distances take 10 us.)
+struct HistConst {
+  double avg, bw;
+  float inv_bw, errc, abs_q, flo, fhi, s_hi;
+};
+static float float_up(double x) {
+  float f = (float)x;
+  if ((double)f < x) f = std::nextafterf(f, HUGE_VALF);
+  return f;
+}
+static HistConst hist_const(double avg, uint32_t d, uint32_t b_lo, uint32_t b_hi, double abs_err) {
+  HistConst c;
+  c.avg = avg;
+  c.bw = avg / (NBUCKETS * 1.0);  // GPU.cu:3356
+  c.inv_bw = (float)(1.0 / c.bw);
+  c.errc = (float)(2 * d + 8) * 5.9604645e-8f;  // (2d+8) * 2^-24, relative
+  c.abs_q = (float)(abs_err / c.bw) * 1.0001f + 1e-4f;
+  c.flo = (float)b_lo;
+  c.fhi = (float)b_hi;
+  // squared-distance prefilter: a pair whose float squared distance is at
+  // least s_hi has q32 - del >= fhi (the kernel's bracket puts it above the
+  // counted range) -- q32 is within 2^-23 of sqrt(s32) / bw, and s_hi is
+  // widened by 2^-20 for its own rounding -- so it is skipped without a root
+  const double q_need = ((double)c.fhi + (double)c.abs_q) / (1.0 - (double)c.errc);
+  const double sq_bw = q_need * c.bw / ((1.0 - 1.0 / 8388608.0) * (1.0 - 1.0 / 8388608.0));
+  c.s_hi = float_up(sq_bw * sq_bw * (1.0 + 1.0 / 1048576.0));
+  return c;
+}
+
+// Counts the buckets in [b_lo, b_hi) of sample blocks.  The brackets use the
+// float columns soaf; abs_err (in the constants) bounds the distance error
+// from rounding the coordinates to float (0 for float data).
 template <typename T>
-__global__ void __launch_bounds__(EPS_BLOCK) eps_hist_kernel(const T* __restrict__ soa, uint64_t n, uint32_t d,
-                                                             uint32_t offset, const double* __restrict__ avg_in,
-                                                             uint32_t* __restrict__ hist, uint32_t b_lo,
-                                                             uint32_t b_hi, double abs_err) {
+__global__ void __launch_bounds__(EPS_BLOCK) eps_hist_kernel(const T* __restrict__ soa,
+                                                             const float* __restrict__ soaf, uint64_t n, uint32_t d,
+                                                             uint32_t offset, uint32_t* __restrict__ hist,
+                                                             uint32_t b_lo, uint32_t b_hi, const HistConst hc) {
   extern __shared__ uint32_t sh[];  // the b_hi - b_lo counted buckets
   const uint32_t nb = b_hi - b_lo;
   for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) sh[i] = 0;
   __syncthreads();
-  const double avg = avg_in[0];
-  const double bw = __ddiv_rn(avg, NBUCKETS * 1.0);  // GPU.cu:3356
+  const double avg = hc.avg, bw = hc.bw;
   // HIST_SPLIT blocks share one sample point, each taking every
   // HIST_SPLIT-th round of candidates (integer counts: the order of the
   // additions does not matter)
   const uint64_t sid = (uint64_t)(blockIdx.x / HIST_SPLIT) * offset;
   const uint32_t part = blockIdx.x % HIST_SPLIT;
-  const float inv_bw = (float)(1.0 / bw);
-  const float errc = (float)(2 * d + 8) * 5.9604645e-8f;  // (2d+8) * 2^-24, relative
-  const float abs_q = (float)(abs_err / bw) * 1.0001f + 1e-4f;
-  const float flo = (float)b_lo, fhi = (float)b_hi;
-  // squared-distance prefilter: a pair whose float squared distance is at
-  // least s_hi has q32 - del >= fhi (the bracket below puts it above the
-  // counted range) -- q32 is within 2^-23 of sqrt(s32) / bw, and s_hi is
-  // widened by 2^-20 for its own rounding -- so it is skipped without a root
-  const double q_need = ((double)fhi + (double)abs_q) / (1.0 - (double)errc);
-  const double sq_bw = q_need * bw / ((1.0 - 1.0 / 8388608.0) * (1.0 - 1.0 / 8388608.0));
-  const float s_hi = __double2float_ru(sq_bw * sq_bw * (1.0 + 1.0 / 1048576.0));
+  const float inv_bw = hc.inv_bw, errc = hc.errc, abs_q = hc.abs_q, flo = hc.flo, fhi = hc.fhi, s_hi = hc.s_hi;
   // the sample point's coordinates once per block; four candidates per
   // thread and round so that their loads overlap
   __shared__ T qs[MAX_D];
-  for (uint32_t l = threadIdx.x; l < d; l += blockDim.x) qs[l] = soa[(uint64_t)l * n + sid];
+  __shared__ float qsf[MAX_D];
+  for (uint32_t l = threadIdx.x; l < d; l += blockDim.x) {
+    qs[l] = soa[(uint64_t)l * n + sid];
+    qsf[l] = soaf[(uint64_t)l * n + sid];
+  }
   __syncthreads();
   constexpr uint64_t STEP = (uint64_t)EPS_BLOCK * 8;
   constexpr int U = 4;
@@ -189,12 +216,12 @@ __global__ void __launch_bounds__(EPS_BLOCK) eps_hist_kernel(const T* __restrict
 #pragma unroll
     for (int u = 0; u < U; u++) s4[u] = 0.0f;
     for (uint32_t l = 0; l < d; l++) {
-      const float qf = (float)qs[l];
+      const float qf = qsf[l];
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const uint64_t p = i0 + u * STEP + threadIdx.x;
         if (p < n) {
-          const float df = __fsub_rn((float)soa[(uint64_t)l * n + p], qf);
+          const float df = __fsub_rn(soaf[(uint64_t)l * n + p], qf);
           s4[u] = __fadd_rn(s4[u], __fmul_rn(df, df));
         }
       }
@@ -272,24 +299,24 @@ void launch_eps_avg(const T* soa, uint64_t n, uint32_t d, const EpsScratch& sc, 
 }
 
 template <typename T>
-void launch_eps_hist(const T* soa, uint64_t n, uint32_t d, const EpsScratch& sc, uint32_t b_lo, uint32_t b_hi,
-                     double abs_err, cudaStream_t s) {
+void launch_eps_hist(const T* soa, const float* soaf, uint64_t n, uint32_t d, const EpsScratch& sc, double avg,
+                     uint32_t b_lo, uint32_t b_hi, double abs_err, cudaStream_t s) {
   const uint32_t offset = eps_sample_offset(n);
   const uint32_t blocks2 = (uint32_t)n / offset;  // GPU.cu:3440 (integer division)
   if (blocks2 > 0 && b_hi > b_lo) {
     // shared memory for the counted bucket range only (256 buckets on the
     // first try: a small footprint lets more blocks share an SM)
     eps_hist_kernel<T><<<blocks2 * HIST_SPLIT, EPS_BLOCK, (size_t)(b_hi - b_lo) * 4, s>>>(
-        soa, n, d, offset, sc.avg_out, sc.hist, b_lo, b_hi, abs_err);
+        soa, soaf, n, d, offset, sc.hist, b_lo, b_hi, hist_const(avg, d, b_lo, b_hi, abs_err));
     KNNSJ_CHECK_LAUNCH();
   }
 }
 
 template void launch_eps_avg<float>(const float*, uint64_t, uint32_t, const EpsScratch&, cudaStream_t);
 template void launch_eps_avg<double>(const double*, uint64_t, uint32_t, const EpsScratch&, cudaStream_t);
-template void launch_eps_hist<float>(const float*, uint64_t, uint32_t, const EpsScratch&, uint32_t, uint32_t,
-                                     double, cudaStream_t);
-template void launch_eps_hist<double>(const double*, uint64_t, uint32_t, const EpsScratch&, uint32_t, uint32_t,
-                                      double, cudaStream_t);
+template void launch_eps_hist<float>(const float*, const float*, uint64_t, uint32_t, const EpsScratch&, double,
+                                     uint32_t, uint32_t, double, cudaStream_t);
+template void launch_eps_hist<double>(const double*, const float*, uint64_t, uint32_t, const EpsScratch&, double,
+                                      uint32_t, uint32_t, double, cudaStream_t);
 
 }  // namespace knnsj

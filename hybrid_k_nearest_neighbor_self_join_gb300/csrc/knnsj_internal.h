@@ -76,7 +76,8 @@ struct DeviceGrid {
 
 // ---- kernel launchers (k_*.cu) -------------------------------------------
 template <typename T>
-void launch_transpose_reorder(const T* aos, T* soa, uint64_t n, uint32_t d, const uint32_t* d_perm,
+// (soaf, optional: the columns rounded to float as well)
+void launch_transpose_reorder(const T* aos, T* soa, float* soaf, uint64_t n, uint32_t d, const uint32_t* d_perm,
                               cudaStream_t s, uint32_t* d_nonfinite);
 template <typename T>
 void launch_minmax(const T* soa, uint64_t n, uint32_t di, T* d_minmax /*2*di*/, T* scratch /*1024*2*di*/,
@@ -94,8 +95,10 @@ uint32_t eps_sample_offset(uint64_t n);
 template <typename T>
 void launch_eps_avg(const T* soa, uint64_t n, uint32_t d, const EpsScratch& sc, cudaStream_t s);
 template <typename T>
-void launch_eps_hist(const T* soa, uint64_t n, uint32_t d, const EpsScratch& sc, uint32_t b_lo, uint32_t b_hi,
-                     double abs_err, cudaStream_t s);
+// avg: the sampled mean distance (*avg_out); soaf: the columns rounded to
+// float (float data: the columns themselves).
+void launch_eps_hist(const T* soa, const float* soaf, uint64_t n, uint32_t d, const EpsScratch& sc, double avg,
+                     uint32_t b_lo, uint32_t b_hi, double abs_err, cudaStream_t s);
 // Sum of squared result distances (the reference's verification figure,
 // GPU.cu:3690-3693) in a fixed order; result in *d_out.
 template <typename T>
