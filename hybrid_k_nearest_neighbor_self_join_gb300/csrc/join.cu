@@ -850,14 +850,30 @@ static bool run_graph_passes(Workspace& w, SearchLaunch<T> a, LoopCtl& c, LoopCt
 // blocks of ids during the first pass, nor those with a cap on the passes of
 // the radius schedule, which counts the schedule's own passes, nor double data
 // that the float screen cannot hold (or is told not to: the ring search then
-// takes every distance in double).  From four dimensions on the ring of cells
-// visits several times the points the tree does and most first passes fail
-// (10 M x 6-D: 3150 candidates per query in 10 passes against 2050 in 3).
+// takes every distance in double), nor where a grid search is asked for
+// (tile_search 2 and 3).
+//
+// Whole joins measured on both sides, 2 000 to 3 000 000 points, k = 8, 64 and
+// 120, float and double, BETA 0.025 (ring over tree time):
+//   four and more dimensions: the ring of cells visits several times the
+//     points and most first passes fail; 1.4x (4-D) to 27x (12-D);
+//   three dimensions: 0.98-3.1x, the tile kernel's learned joins included;
+//   two dimensions, a uniform radius: 0.97-2.5x from 30 000 points on (most
+//     first passes fail; the tree needs no schedule of passes), 1.0-1.3x at
+//     2 000 (0.8x at k = 120, where few passes fail);
+//   two dimensions, learned radii: rings of a few cells, few failures.  The
+//     tile kernel (float, k + 1 <= 65) 0.5-0.9x at 3 M; one warp per query
+//     0.9-1.2x below a million points, 1.04-1.36x at 3 M.
+constexpr uint64_t TREE_LEARNED_2D_MIN = 1000000;
 template <typename T>
-static bool tree_applies(const JoinConfig& cfg, uint32_t d, double max_abs, bool will_stream) {
+static bool tree_applies(const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t di, uint32_t K, double max_abs,
+                         bool will_stream) {
   if (!cfg.tree_search || will_stream || cfg.max_iterations > 0) return false;
   if (sizeof(T) == 8 && (!cfg.float_prefilter || !(4.0 * std::sqrt((double)d) * max_abs < 1e18))) return false;
-  return cfg.tree_search == 2 || d >= 4;
+  if (cfg.tree_search == 2) return true;
+  if (cfg.tile_search >= 2) return false;
+  if (d >= 3 || cfg.radius_mode != KNNSJ_RADIUS_LEARNED) return true;
+  return n >= TREE_LEARNED_2D_MIN && !(cfg.tile_search && tile_search_applies(d, di, K, 1, sizeof(T)));
 }
 
 struct TreePasses {
@@ -966,7 +982,7 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
   rec(1);
 
   const bool will_stream = rows && rows->chunks >= 2 && n >= (uint64_t)rows->chunks;
-  const bool use_tree = tree_applies<T>(cfg, d, P.max_abs, will_stream);
+  const bool use_tree = tree_applies<T>(cfg, n, d, di, K, P.max_abs, will_stream);
   // 5. starting radii: eps0 for every query (plain), or one per query
   T* qrad = nullptr;
   double rmax = (double)P.eps0;
