@@ -878,7 +878,7 @@ knnsj_status knnsj_radius_grad(const float* model, const float* features, const 
         float* dt = (float*)w.ids.get(n * 4);
         const size_t np = mlp_grad_partials(n);
         float* dpart = (float*)w.dists.get(np * 4);
-        double* dpl = (double*)w.eps_partial.get(((n + 63) / 64) * 8);
+        double* dpl = (double*)w.eps_partial.get((size_t)mlp_grad_blocks(n) * 8);
         float* dg = (float*)w.eps_sample.get(KNNSJ_RADIUS_MODEL_FLOATS * 4);
         KNNSJ_CUDA(cudaMemcpyAsync(dm, model, KNNSJ_RADIUS_MODEL_FLOATS * 4, cudaMemcpyHostToDevice, s));
         KNNSJ_CUDA(cudaMemcpyAsync(df, features, n * KNNSJ_RADIUS_FEATURES * 4, cudaMemcpyHostToDevice, s));
@@ -886,7 +886,7 @@ knnsj_status knnsj_radius_grad(const float* model, const float* features, const 
         mlp_grad_device(dm, df, dt, nullptr, n, quantile, 1.0f / (float)n, dpart, dpl, dg, s);
         const size_t ntrain = KNNSJ_RADIUS_MODEL_FLOATS - 2 * KNNSJ_RADIUS_FEATURES;
         KNNSJ_CUDA(cudaMemcpyAsync(out_grad, dg, ntrain * 4, cudaMemcpyDeviceToHost, s));
-        std::vector<double> pl((n + 63) / 64);
+        std::vector<double> pl(mlp_grad_blocks(n));
         KNNSJ_CUDA(cudaMemcpyAsync(pl.data(), dpl, pl.size() * 8, cudaMemcpyDeviceToHost, s));
         KNNSJ_CUDA(cudaStreamSynchronize(s));
         if (out_loss) {

@@ -386,7 +386,8 @@ void radius_model_set(const float* model);  // nullptr restores the built-in mod
 void mlp_grad_device(const float* d_model, const float* d_X, const float* d_Y, const uint32_t* d_idx, uint64_t n,
                      float quantile, float inv_batch, float* d_part, double* d_part_loss, float* d_grad,
                      cudaStream_t s);
-size_t mlp_grad_partials(uint64_t n);  // floats of d_part for n samples
+uint32_t mlp_grad_blocks(uint64_t n);  // elements of d_part_loss for n samples
+size_t mlp_grad_partials(uint64_t n);  // floats of d_part
 void train_model(const float* hX, const float* hY, uint64_t n, int epochs, uint32_t batch, float lr,
                  float quantile, uint64_t seed, float* model_out, float* loss_out, cudaStream_t s);
 
