@@ -156,10 +156,13 @@ void Workspace::ensure_copy_stream() {
   if (!copy_stream) KNNSJ_CUDA(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
   for (auto& e : chunk_ev)
     if (!e) KNNSJ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  if (!mail_host) {
-    KNNSJ_CUDA(cudaHostAlloc(&mail_host, MAIL_BYTES, cudaHostAllocMapped));
-    KNNSJ_CUDA(cudaHostGetDevicePointer(&mail_dev, mail_host, 0));
-  }
+  ensure_mail();
+}
+
+void Workspace::ensure_mail() {
+  if (mail_host || g_forbid_alloc) return;  // (fixed-scratch joins copy into pageable memory)
+  KNNSJ_CUDA(cudaHostAlloc(&mail_host, MAIL_BYTES, cudaHostAllocMapped));
+  KNNSJ_CUDA(cudaHostGetDevicePointer(&mail_dev, mail_host, 0));
 }
 
 namespace {
@@ -230,17 +233,57 @@ static void dev_copy(Workspace& w, void* dst, const void* src, size_t bytes, cud
     KNNSJ_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, s));
 }
 
-// Device-to-host read of a few bytes (a multiple of 4); synchronises s.
-static void read_small(Workspace& w, void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  if (w.mail) {
-    if (bytes > MAIL_BYTES / 2) throw StatusError{KNNSJ_ERR_UNSUPPORTED, "mailbox read too large"};
-    launch_copy_words(w.mail_dev, src, bytes, s);
+// One piece of a device-to-host read (a multiple of 4 bytes).
+struct Piece {
+  void* dst;
+  const void* src;
+  size_t bytes;
+};
+namespace {
+constexpr int MAX_PIECES = 4;
+struct PieceList {
+  const uint32_t* src[MAX_PIECES];
+  uint32_t words[MAX_PIECES];
+};
+// Gathers the pieces one after the other at dst (mapped host memory).
+__global__ void __launch_bounds__(1024) collect_kernel(uint32_t* __restrict__ dst, const PieceList l) {
+  uint32_t at = 0;
+  for (int p = 0; p < MAX_PIECES; p++) {
+    for (uint32_t i = threadIdx.x; i < l.words[p]; i += blockDim.x) dst[at + i] = l.src[p][i];
+    at += l.words[p];
+  }
+}
+}  // namespace
+
+// Device-to-host reads of a few small pieces with one synchronisation of s.
+static void read_pieces(Workspace& w, std::initializer_list<Piece> pieces, cudaStream_t s) {
+  size_t bytes = 0;
+  for (const Piece& p : pieces) bytes += p.bytes;
+  w.ensure_mail();
+  if (w.mail_host && bytes <= MAIL_BYTES / 2 && pieces.size() <= MAX_PIECES) {
+    PieceList l{};
+    int i = 0;
+    for (const Piece& p : pieces) {
+      l.src[i] = (const uint32_t*)p.src;
+      l.words[i++] = (uint32_t)(p.bytes / 4);
+    }
+    collect_kernel<<<1, bytes > 1024 ? 1024 : 128, 0, s>>>((uint32_t*)w.mail_dev, l);
+    KNNSJ_CHECK_LAUNCH();
     KNNSJ_CUDA(cudaStreamSynchronize(s));
-    std::memcpy(dst, w.mail_host, bytes);
+    const unsigned char* at = (const unsigned char*)w.mail_host;
+    for (const Piece& p : pieces) {
+      std::memcpy(p.dst, at, p.bytes);
+      at += p.bytes;
+    }
     return;
   }
-  KNNSJ_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+  if (w.mail) throw StatusError{KNNSJ_ERR_UNSUPPORTED, "mailbox read too large"};
+  for (const Piece& p : pieces) KNNSJ_CUDA(cudaMemcpyAsync(p.dst, p.src, p.bytes, cudaMemcpyDeviceToHost, s));
   KNNSJ_CUDA(cudaStreamSynchronize(s));
+}
+
+static void read_small(Workspace& w, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  read_pieces(w, {Piece{dst, src, bytes}}, s);
 }
 
 // Host-to-device write of a few bytes (a multiple of 4); the source may be
@@ -260,24 +303,31 @@ static void write_small(Workspace& w, void* dst, const void* src, size_t bytes, 
 
 namespace {
 
-struct SmallDev {  // layout of Workspace::small
+// What the host reads of a join (cleared when the join starts).
+struct SmallHead {
   uint32_t nonfinite;
   uint32_t fail_count;
   uint32_t work_counter;
-  uint32_t defer_count;  // queries the tile search handed to search_kernel (current launch)
-  unsigned long long C;
+  uint32_t defer_count;                 // queries the tile search handed to search_kernel (current launch)
+  unsigned long long C0;                // non-empty cells of the eps0 grid
   unsigned long long cand;
   double avg[2];
-  uint32_t hist[10000];
+  unsigned long long defer_total;       // all queries handed over by the tile search in this join
+  unsigned long long tree_rmax;         // tree search: largest radius grown or searched (bits)
+  uint32_t tree_fail[2];                // tree search: failures of its first two passes
+  uint32_t mlp_err;                     // the tensor-core radius MLP timed out
+  uint32_t pad;
   double csum;
+};
+struct SmallDev : SmallHead {  // layout of Workspace::small
+  uint32_t hist[HIST_BUCKETS];
+  unsigned long long C;                 // non-empty cells of a rebuilt grid
+  HistConst hc[2];
   double cpart[1024];
   FailRadii fr;
   LoopCtl ctl;
-  uint32_t mlp_err;  // the tensor-core radius MLP timed out
   uint32_t chunk_fill[MAX_ROW_CHUNKS];  // streamed rows: queries placed per id block
   uint32_t patch_count;                 // streamed rows: first-pass failures
-  uint32_t tree_fail[2];                // tree search: failures of its first two passes
-  unsigned long long defer_total;       // all queries handed over by the tile search in this join
 };
 
 template <typename T>
@@ -291,11 +341,9 @@ T host_fallback_eps(const std::vector<T>& mn, const std::vector<T>& mx, uint64_t
 
 }  // namespace
 
+// generateNDGridDimensions (main.cu:2425-2488), in DTYPE.
 template <typename T>
-static void build_grid(Workspace& w, const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t di,
-                       const std::vector<T>& mn, const std::vector<T>& mx, T width, DeviceGrid<T>* out,
-                       cudaStream_t s) {
-  // generateNDGridDimensions (main.cu:2425-2488), in DTYPE.
+static GridGeom<T> grid_geometry(uint32_t di, const std::vector<T>& mn, const std::vector<T>& mx, T width) {
   GridGeom<T> g{};
   g.di = di;
   g.width = width;
@@ -315,8 +363,17 @@ static void build_grid(Workspace& w, const JoinConfig& cfg, uint64_t n, uint32_t
   }
   if (overflow) throw StatusError{KNNSJ_ERR_UNSUPPORTED, "more than 2^64 grid cells"};
   g.total_cells = mult;
+  return g;
+}
+
+// The grid index of width `width`; d_C receives its number of non-empty cells.
+template <typename T>
+static void build_grid(Workspace& w, const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t di,
+                       const std::vector<T>& mn, const std::vector<T>& mx, T width, unsigned long long* d_C,
+                       DeviceGrid<T>* out, cudaStream_t s) {
+  const GridGeom<T> g = grid_geometry<T>(di, mn, mx, width);
   int bits = 0;
-  while (bits < 64 && ((mult - 1) >> bits) != 0) bits++;
+  while (bits < 64 && ((g.total_cells - 1) >> bits) != 0) bits++;
 
   GridScratch sc;
   sc.keys[0] = (unsigned long long*)w.keys0.get(n * 8);
@@ -336,23 +393,20 @@ static void build_grid(Workspace& w, const JoinConfig& cfg, uint64_t n, uint32_t
   uint32_t* pos = (uint32_t*)w.pos.get(n * 4);
   unsigned long long* ckeys = (unsigned long long*)w.ckeys.get(n * 8);
   uint32_t* coff = (uint32_t*)w.coff.get((n + 1) * 4);
-  SmallDev* sm = (SmallDev*)w.small.p;
-  launch_compact_cells(skeys, n, flags, pos, sc.scan_tmp, ckeys, coff, &sm->C, s);
+  launch_compact_cells(skeys, n, flags, pos, sc.scan_tmp, ckeys, coff, d_C, s);
   // (the box tree keeps its columns in the same buffers, at its own stride)
   T* ps = (T*)w.ps.get(tree_stride(n) * d * sizeof(T));
   float* psf = sizeof(T) == 8 ? (float*)w.psf.get(tree_stride(n) * d * sizeof(float)) : nullptr;
   uint32_t* pid = (uint32_t*)w.pid.get(n * 4);
   dev_copy(w, pid, sids, n * 4, s);
   launch_gather_sorted<T>(xs, n, d, sids, ps, psf, s);
-  unsigned long long C = 0;
-  read_small(w, &C, &sm->C, sizeof(C), s);
   out->geom = g;
   out->ps = ps;
   out->psf = psf;
   out->pid = pid;
   out->ckeys = ckeys;
   out->coff = coff;
-  out->C = C;
+  out->C = 0;
   const unsigned long long dense_limit =
       cfg.dense_cells_cap ? cfg.dense_cells_cap : std::max<unsigned long long>(4ull * n, 1ull << 24);
   out->dense = (cfg.dense_mode != 0) && (g.total_cells <= dense_limit) && g.total_cells < (1ull << 31);
@@ -361,8 +415,10 @@ static void build_grid(Workspace& w, const JoinConfig& cfg, uint64_t n, uint32_t
   out->dstart = nullptr;
   if (out->dense) {
     uint32_t* dstart = (uint32_t*)w.dstart.get((g.total_cells + 1) * 4);
-    launch_dense_table(ckeys, coff, C, g.total_cells, dstart, s);
+    launch_dense_table(ckeys, coff, d_C, g.total_cells, dstart, s);
     out->dstart = dstart;
+  } else {  // the searches of the cell list take its length
+    read_small(w, &out->C, d_C, sizeof(out->C), s);
   }
 }
 
@@ -615,9 +671,40 @@ struct Prepared {
   std::vector<T> mn, mx;
 };
 
+// Joins searched through the box tree.  Not those whose rows stream out in
+// blocks of ids during the first pass, nor those with a cap on the passes of
+// the radius schedule, which counts the schedule's own passes, nor double data
+// that the float screen cannot hold (or is told not to: the ring search then
+// takes every distance in double), nor where a grid search is asked for
+// (tile_search 2 and 3).
+//
+// Whole joins measured on both sides, 2 000 to 3 000 000 points, k = 8, 64 and
+// 120, float and double, BETA 0.025 (ring over tree time):
+//   four and more dimensions: the ring of cells visits several times the
+//     points and most first passes fail; 1.4x (4-D) to 27x (12-D);
+//   three dimensions: 0.98-3.1x, the tile kernel's learned joins included;
+//   two dimensions, a uniform radius: 0.97-2.5x from 30 000 points on (most
+//     first passes fail; the tree needs no schedule of passes), 1.0-1.3x at
+//     2 000 (0.8x at k = 120, where few passes fail);
+//   two dimensions, learned radii: rings of a few cells, few failures.  The
+//     tile kernel (float, k + 1 <= 65) 0.5-0.9x at 3 M; one warp per query
+//     0.9-1.2x below a million points, 1.04-1.36x at 3 M.
+constexpr uint64_t TREE_LEARNED_2D_MIN = 1000000;
+template <typename T>
+static bool tree_applies(const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t di, uint32_t K, double max_abs,
+                         bool will_stream) {
+  if (!cfg.tree_search || will_stream || cfg.max_iterations > 0) return false;
+  if (sizeof(T) == 8 && (!cfg.float_prefilter || !(4.0 * std::sqrt((double)d) * max_abs < 1e18))) return false;
+  if (cfg.tree_search == 2) return true;
+  if (cfg.tile_search >= 2) return false;
+  if (d >= 3 || cfg.radius_mode != KNNSJ_RADIUS_LEARNED) return true;
+  return n >= TREE_LEARNED_2D_MIN && !(cfg.tile_search && tile_search_applies(d, di, K, 1, sizeof(T)));
+}
+
 template <typename T>
 static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_aos, uint64_t n, uint32_t d,
-                    uint32_t k, knnsj_stats* st, cudaStream_t s, Prepared<T>* P) {
+                    uint32_t k, knnsj_stats* st, cudaStream_t s, Prepared<T>* P, bool will_stream = false,
+                    bool* use_tree = nullptr) {
   const uint32_t K = k + 1;
   const uint32_t di = cfg.num_indexed_dims;
 
@@ -626,72 +713,75 @@ static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T
   for (uint32_t j = 0; j < d; j++) perm[j] = j;
   if (!cfg.no_reorder) {
     const uint64_t ns = (n + 99) / 100;
-    std::vector<T> sample(ns * d);
+    std::vector<T> sample;
+    const T* sp = nullptr;
     if (h_aos) {
+      sample.resize(ns * d);
       for (uint64_t i = 0; i < ns; i++)
         std::memcpy(&sample[i * d], h_aos + i * 100 * d, d * sizeof(T));
+      sp = sample.data();
+    } else if (!g_forbid_alloc) {
+      // gathered by a kernel straight into mapped memory (a strided copy of
+      // rows of a few bytes is slow on the copy engines)
+      T* host = (T*)w.pinned(ns * d * sizeof(T));
+      void* dev = nullptr;
+      KNNSJ_CUDA(cudaHostGetDevicePointer(&dev, host, 0));
+      launch_gather_rows<T>(d_aos, ns, 100, d, (T*)dev, s);
+      KNNSJ_CUDA(cudaStreamSynchronize(s));
+      sp = host;
     } else {
+      sample.resize(ns * d);
       KNNSJ_CUDA(cudaMemcpy2DAsync(sample.data(), d * sizeof(T), d_aos, 100 * d * sizeof(T),
                                    d * sizeof(T), ns, cudaMemcpyDeviceToHost, s));
       KNNSJ_CUDA(cudaStreamSynchronize(s));
+      sp = sample.data();
     }
-    reorder_from_sample<T>(sample.data(), ns, n, d, perm.data(), nullptr);
+    reorder_from_sample<T>(sp, ns, n, d, perm.data(), nullptr);
   }
   if (st)
     for (uint32_t j = 0; j < d && j < 64; j++) st->perm[j] = perm[j];
 
   // 2. transpose into column arrays
-  uint32_t* d_perm = (uint32_t*)w.perm.get(d * 4);
   SmallDev* sm = (SmallDev*)w.small.get(sizeof(SmallDev));
-  KNNSJ_CUDA(cudaMemsetAsync(sm, 0, offsetof(SmallDev, hist), s));
-  launch_zero_words(&sm->defer_total, sizeof(sm->defer_total), s);
-  KNNSJ_CUDA(cudaMemcpyAsync(d_perm, perm.data(), d * 4, cudaMemcpyHostToDevice, s));
+  KNNSJ_CUDA(cudaMemsetAsync(sm, 0, offsetof(SmallDev, C), s));  // the head and the histogram
   T* xs = (T*)w.xs.get(n * d * sizeof(T));
   // (double data: a float copy too, for the histogram's brackets; the buffer
   // later holds the cell-ordered float columns)
   float* xsf = sizeof(T) == 8 ? (float*)w.psf.get(tree_stride(n) * d * sizeof(float)) : nullptr;
-  launch_transpose_reorder<T>(d_aos, xs, xsf, n, d, d_perm, s, &sm->nonfinite);
+  launch_transpose_reorder<T>(d_aos, xs, xsf, n, d, perm.data(), s, &sm->nonfinite);
   if (!xsf) xsf = reinterpret_cast<float*>(xs);
   T* mm_part = (T*)w.minmax_part.get(1024 * 2 * d * sizeof(T) + 2 * d * sizeof(T));
   T* d_minmax = mm_part + 1024 * 2 * d;
   launch_minmax<T>(xs, n, d, d_minmax, mm_part, s);
 
-  // 3. eps0 (GPU.cu:3088-3566)
+  // 3. eps0 (GPU.cu:3088-3566): the mean distance and the first range of the
+  // histogram, then one look at the results (the rest of the histogram only if
+  // the crossing lies beyond)
   EpsScratch es;
   const uint64_t nthr = eps_avg_threads(n);
   es.partial = (double*)w.eps_partial.get(std::max<uint64_t>(nthr * eps_avg_chunks(n), 1) * 8);
   es.sample_sum = (double*)w.eps_sample.get(std::max<uint64_t>(nthr, 1) * 8);
   es.avg_out = sm->avg;
   es.hist = sm->hist;
-  launch_eps_avg<T>(xs, n, d, es, s);
-  KNNSJ_CUDA(cudaMemsetAsync(sm->hist, 0, sizeof(sm->hist), s));
-  struct Head {
-    uint32_t nonfinite, fail_count, work_counter, defer_count;
-    unsigned long long C, cand;
-    double avg[2];
-  } head;
+  es.hc = sm->hc;
+  launch_eps_avg<T>(xs, d_minmax, n, d, es, s);
+  launch_eps_hist<T>(xs, xsf, n, d, es, 0, s);
+  SmallHead head;
   std::vector<T> hmm(2 * d);
-  KNNSJ_CUDA(cudaMemcpyAsync(hmm.data(), d_minmax, 2 * d * sizeof(T), cudaMemcpyDeviceToHost, s));
-  KNNSJ_CUDA(cudaMemcpyAsync(&head, sm, sizeof(head), cudaMemcpyDeviceToHost, s));
-  KNNSJ_CUDA(cudaStreamSynchronize(s));
+  std::vector<uint32_t> hh(HIST_BUCKETS, 0);
+  read_pieces(w, {Piece{&head, static_cast<SmallHead*>(sm), sizeof(head)},
+                  Piece{hh.data(), sm->hist, HIST_FIRST * 4},
+                  Piece{hmm.data(), d_minmax, 2 * d * sizeof(T)}}, s);
   if (head.nonfinite) throw StatusError{KNNSJ_ERR_NONFINITE_INPUT, "NaN or infinite coordinate"};
-  // float bracket error from rounding double coordinates to float
   double max_abs = 0.0;
   for (uint32_t j = 0; j < 2 * d; j++) max_abs = std::max(max_abs, std::fabs((double)hmm[j]));
-  const double abs_err = sizeof(T) == 8 ? std::sqrt((double)d) * std::ldexp(max_abs, -22) : 0.0;
   P->max_abs = max_abs;
-  // buckets [0, 256) first; the rest only if the crossing lies beyond
-  std::vector<uint32_t> hh(10000, 0);
-  const uint32_t first_range = 256;
-  launch_eps_hist<T>(xs, xsf, n, d, es, head.avg[0], 0, first_range, abs_err, s);
-  KNNSJ_CUDA(cudaMemcpyAsync(hh.data(), sm->hist, first_range * 4, cudaMemcpyDeviceToHost, s));
-  KNNSJ_CUDA(cudaStreamSynchronize(s));
-  EpsChoice ec = choose_eps(hh.data(), first_range, head.avg[0], n, k, cfg.beta);
+  EpsChoice ec = choose_eps(hh.data(), HIST_FIRST, head.avg[0], n, k, cfg.beta);
   if (!ec.complete) {
-    launch_eps_hist<T>(xs, xsf, n, d, es, head.avg[0], first_range, 10000, abs_err, s);
-    KNNSJ_CUDA(cudaMemcpyAsync(hh.data(), sm->hist, 10000 * 4, cudaMemcpyDeviceToHost, s));
+    launch_eps_hist<T>(xs, xsf, n, d, es, 1, s);
+    KNNSJ_CUDA(cudaMemcpyAsync(hh.data(), sm->hist, HIST_BUCKETS * 4, cudaMemcpyDeviceToHost, s));
     KNNSJ_CUDA(cudaStreamSynchronize(s));
-    ec = choose_eps(hh.data(), 10000, head.avg[0], n, k, cfg.beta);
+    ec = choose_eps(hh.data(), HIST_BUCKETS, head.avg[0], n, k, cfg.beta);
   }
   T eps0 = (T)ec.eps;
   P->mn.assign(di, 0);
@@ -718,9 +808,20 @@ static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T
     st->avg_distance = head.avg[0];
   }
 
-  // 4. grid at eps0
-  build_grid<T>(w, cfg, n, d, di, P->mn, P->mx, eps0, &P->grid, s);
-  if (st) st->nonempty_cells = P->grid.C;
+  // 4. grid at eps0.  A box-tree search with a uniform radius does not read it:
+  // its cells are only counted, where a bitmap of them fits (up to 32 MB, or
+  // what the fixed scratch array grants a dense table).
+  if (use_tree) *use_tree = tree_applies<T>(cfg, n, d, di, k + 1, max_abs, will_stream);
+  if (use_tree && *use_tree && cfg.radius_mode != KNNSJ_RADIUS_LEARNED) {
+    const GridGeom<T> g = grid_geometry<T>(di, P->mn, P->mx, eps0);
+    P->grid.geom = g;
+    const unsigned long long cap = cfg.dense_cells_cap ? 32ull * cfg.dense_cells_cap : 1ull << 28;
+    if (g.total_cells <= cap) {
+      launch_count_cells<T>(xs, n, g, (uint32_t*)w.dstart.get((size_t)((g.total_cells + 31) / 32) * 4), &sm->C0, s);
+      return;
+    }
+  }
+  build_grid<T>(w, cfg, n, d, di, P->mn, P->mx, eps0, &sm->C0, &P->grid, s);
 }
 
 // The radius model used by the learned starting radius, uploaded to the
@@ -846,49 +947,12 @@ static bool run_graph_passes(Workspace& w, SearchLaunch<T> a, LoopCtl& c, LoopCt
   return true;
 }
 
-// Joins searched through the box tree.  Not those whose rows stream out in
-// blocks of ids during the first pass, nor those with a cap on the passes of
-// the radius schedule, which counts the schedule's own passes, nor double data
-// that the float screen cannot hold (or is told not to: the ring search then
-// takes every distance in double), nor where a grid search is asked for
-// (tile_search 2 and 3).
-//
-// Whole joins measured on both sides, 2 000 to 3 000 000 points, k = 8, 64 and
-// 120, float and double, BETA 0.025 (ring over tree time):
-//   four and more dimensions: the ring of cells visits several times the
-//     points and most first passes fail; 1.4x (4-D) to 27x (12-D);
-//   three dimensions: 0.98-3.1x, the tile kernel's learned joins included;
-//   two dimensions, a uniform radius: 0.97-2.5x from 30 000 points on (most
-//     first passes fail; the tree needs no schedule of passes), 1.0-1.3x at
-//     2 000 (0.8x at k = 120, where few passes fail);
-//   two dimensions, learned radii: rings of a few cells, few failures.  The
-//     tile kernel (float, k + 1 <= 65) 0.5-0.9x at 3 M; one warp per query
-//     0.9-1.2x below a million points, 1.04-1.36x at 3 M.
-constexpr uint64_t TREE_LEARNED_2D_MIN = 1000000;
-template <typename T>
-static bool tree_applies(const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t di, uint32_t K, double max_abs,
-                         bool will_stream) {
-  if (!cfg.tree_search || will_stream || cfg.max_iterations > 0) return false;
-  if (sizeof(T) == 8 && (!cfg.float_prefilter || !(4.0 * std::sqrt((double)d) * max_abs < 1e18))) return false;
-  if (cfg.tree_search == 2) return true;
-  if (cfg.tile_search >= 2) return false;
-  if (d >= 3 || cfg.radius_mode != KNNSJ_RADIUS_LEARNED) return true;
-  return n >= TREE_LEARNED_2D_MIN && !(cfg.tile_search && tile_search_applies(d, di, K, 1, sizeof(T)));
-}
-
-struct TreePasses {
-  int passes = 1;
-  uint64_t queries_run = 0;
-  double ms = 0.0;    // device time of the search kernels
-  double rmax = 0.0;  // largest radius grown or searched (0: none)
-};
-
 // Builds the tree over the grid's point buffers (the grid is not searched
 // afterwards) and runs the passes: each reads its query count on the device,
 // so nothing waits for the host in between.
 template <typename T>
-static TreePasses run_tree(Workspace& w, const Prepared<T>& P, uint64_t n, uint32_t d,
-                           uint32_t di, uint32_t K, T* qrad, int32_t* d_ids, T* d_dists, double* rowsum, uint32_t* const* list, SmallDev* sm,
+static void run_tree(Workspace& w, const Prepared<T>& P, uint64_t n, uint32_t d,
+                     uint32_t di, uint32_t K, T* qrad, int32_t* d_ids, T* d_dists, double* rowsum, uint32_t* list, SmallDev* sm,
                            cudaStream_t s) {
   BoxTree<T> t;
   tree_shape(n, d, t.count, t.offset, &t.levels, &t.nodes);
@@ -909,9 +973,8 @@ static TreePasses run_tree(Workspace& w, const Prepared<T>& P, uint64_t n, uint3
   sc.sort.scan_tmp = (uint32_t*)w.scan_tmp.get(sc.sort.scan_tmp_elems * 4);
   sc.split = (float*)w.tree_split.get(tree_split_elems() * 4);
   launch_tree_build<T>(P.xs, P.minmax, n, d, sc, t, s);
-  launch_zero_words(sm->tree_fail, sizeof(sm->tree_fail), s);
-  launch_zero_words(&sm->fr, sizeof(FailRadii), s);
-  for (int i = 0; i < 2; i++) launch_zero_words(list[i], (size_t)t.count[0] * 4, s);
+  uint32_t* mask[2] = {list, list + t.count[0]};
+  launch_zero_words(list, (size_t)2 * t.count[0] * 4, s);
   TreeLaunch<T> a;
   a.tree = t;
   a.n = n;
@@ -923,39 +986,25 @@ static TreePasses run_tree(Workspace& w, const Prepared<T>& P, uint64_t n, uint3
   a.out_ids = d_ids;
   a.out_d = d_dists;
   a.rowsum = rowsum;
-  a.fail_mask = list[0];
+  a.fail_mask = mask[0];
   a.fail_count = &sm->tree_fail[0];
   a.grow = (T*)w.qradius.get(n * sizeof(T));
-  a.rmax_bits = &sm->fr.rmax_bits;
+  a.rmax_bits = &sm->tree_rmax;
   a.cand_count = &sm->cand;
   if (w.ev[4]) KNNSJ_CUDA(cudaEventRecord(w.ev[4], s));
   launch_tree_search<T>(a, w.sm_count, s);
-  a.qmask = list[0];
+  a.qmask = mask[0];
   a.nq_dev = &sm->tree_fail[0];
   a.qradius = a.grow;
-  a.fail_mask = list[1];
+  a.fail_mask = mask[1];
   a.fail_count = &sm->tree_fail[1];
   launch_tree_search<T>(a, w.sm_count, s);
-  a.qmask = list[1];
+  a.qmask = mask[1];
   a.nq_dev = &sm->tree_fail[1];
   a.qradius = nullptr;
   a.unbounded = 1;
   launch_tree_search<T>(a, w.sm_count, s);
   if (w.ev[5]) KNNSJ_CUDA(cudaEventRecord(w.ev[5], s));
-  TreePasses r;
-  uint32_t fail[2];
-  unsigned long long bits = 0;
-  read_small(w, fail, sm->tree_fail, sizeof(fail), s);
-  read_small(w, &bits, &sm->fr.rmax_bits, sizeof(bits), s);
-  r.passes = 1 + (fail[0] > 0) + (fail[1] > 0);
-  r.queries_run = n + fail[0] + fail[1];
-  r.rmax = decode_radius<T>(bits);
-  if (w.ev[4] && w.ev[5]) {
-    float ms = 0.f;
-    KNNSJ_CUDA(cudaEventElapsedTime(&ms, w.ev[4], w.ev[5]));
-    r.ms = ms;
-  }
-  return r;
 }
 
 template <typename T>
@@ -977,18 +1026,17 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
   g_launches = 0;
   rec(0);
   Prepared<T> P;
-  prepare<T>(w, cfg, d_aos, h_aos, n, d, k, st, s, &P);
+  const bool will_stream = rows && rows->chunks >= 2 && n >= (uint64_t)rows->chunks;
+  bool use_tree = false;
+  prepare<T>(w, cfg, d_aos, h_aos, n, d, k, st, s, &P, will_stream, &use_tree);
   SmallDev* sm = (SmallDev*)w.small.p;
   rec(1);
 
-  const bool will_stream = rows && rows->chunks >= 2 && n >= (uint64_t)rows->chunks;
-  const bool use_tree = tree_applies<T>(cfg, n, d, di, K, P.max_abs, will_stream);
   // 5. starting radii: eps0 for every query (plain), or one per query
   T* qrad = nullptr;
   double rmax = (double)P.eps0;
   if (cfg.radius_mode == KNNSJ_RADIUS_LEARNED) {
     qrad = (T*)w.qradius.get(n * sizeof(T));
-    KNNSJ_CUDA(cudaMemsetAsync(&sm->mlp_err, 0, 4, s));
     // (a box-tree search does not care how many cells a radius spans)
     const double max_cells = use_tree ? 64.0 : learned_max_cells(di);
     launch_radius_assign<T>(P.grid, n, d, k, (float)cfg.beta, device_model(w, s), (double)P.eps0,
@@ -1177,15 +1225,9 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
   // 6b. the box tree: every query at its starting radius, the failures at a
   // radius grown from what they found, and the rest without a radius
   if (use_tree) {
-    TreePasses tp = run_tree<T>(w, P, n, d, di, K, qrad, d_ids, d_dists, rowsum, list, sm, s);
-    iter = tp.passes;
+    run_tree<T>(w, P, n, d, di, K, qrad, d_ids, d_dists, rowsum, list[0], sm, s);
     regrids = 1;  // the index was rebuilt once, as the tree
-    queries_run = tp.queries_run;
-    kernel_ms += tp.ms;
-    alg_bytes += (double)tp.passes * n * d * sizeof(T) + (double)queries_run * d * sizeof(T) +
-                 (double)n * K * (4.0 + sizeof(T));
-    if (tp.rmax > 0.0) rmax_seen = std::max(qrad ? rmax_seen : 0.0, tp.rmax);
-    nq = 0;
+    nq = 0;       // (the passes are counted from the head below)
   }
 
   while (nq > 0) {
@@ -1218,7 +1260,7 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
       // coarser grid for the radius in flight (like main.cu:333-356); the
       // widened width keeps that radius's ring at three cells per dimension
       const T wnew = (T)(rgrid * (1.0 + 1.0 / 32768.0));
-      build_grid<T>(w, cfg, n, d, di, P.mn, P.mx, wnew, &a.grid, s);
+      build_grid<T>(w, cfg, n, d, di, P.mn, P.mx, wnew, &sm->C, &a.grid, s);
       r_limit = regrid_limit((double)a.grid.geom.width, di);
       regrids++;
     }
@@ -1316,15 +1358,20 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
     w.mail = false;
     if (rows->checksum) read_small(w, &rows->total_distance, &sm->csum, sizeof(double), s);
   }
-  if (rowsum && st) {
-    launch_sum_f64(rowsum, n, sm->cpart, &sm->csum, s);
-    read_small(w, &st->total_distance, &sm->csum, sizeof(double), s);
+  if (rowsum && st) launch_sum_f64(rowsum, n, sm->cpart, &sm->csum, s);
+  SmallHead head;
+  read_small(w, &head, static_cast<SmallHead*>(sm), sizeof(head), s);
+  if (rowsum && st) st->total_distance = head.csum;
+  const unsigned long long cand = head.cand;
+  const uint32_t mlp_err = qrad ? head.mlp_err : 0u;
+  if (use_tree) {
+    iter = 1 + (head.tree_fail[0] > 0) + (head.tree_fail[1] > 0);
+    queries_run = n + head.tree_fail[0] + head.tree_fail[1];
+    kernel_ms += elapsed(4, 5);
+    alg_bytes += (double)iter * n * d * sizeof(T) + (double)queries_run * d * sizeof(T) +
+                 (double)n * K * (4.0 + sizeof(T));
+    rmax_seen = std::max(qrad ? rmax_seen : (double)r, decode_radius<T>(head.tree_rmax));
   }
-  unsigned long long cand = 0, deferred = 0;
-  uint32_t mlp_err = 0;
-  read_small(w, &cand, &sm->cand, 8, s);
-  read_small(w, &deferred, &sm->defer_total, 8, s);
-  if (qrad) read_small(w, &mlp_err, &sm->mlp_err, 4, s);
   if (mlp_err && cfg.verbose)  // rows are still exact: the affected queries started at eps0
     fprintf(stderr, "knnsj: the tensor-core radius model timed out (%u); those queries started at eps0\n", mlp_err);
   if (st) {
@@ -1338,7 +1385,8 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
     st->search_alg_bytes = alg_bytes;
     st->search_alg_flops = 3.0 * d * (double)cand;
     st->radius_model_error = (double)mlp_err;
-    st->tile_handovers = (double)deferred;
+    st->tile_handovers = (double)head.defer_total;
+    st->nonempty_cells = head.C0;
     const float a01 = elapsed(0, 1), a12 = elapsed(1, 2);
     st->ms_prep = a01;
     st->ms_search = a12;

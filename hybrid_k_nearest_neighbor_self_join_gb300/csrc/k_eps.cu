@@ -36,7 +36,7 @@ namespace knnsj {
 namespace {
 
 constexpr int EPS_BLOCK = 256;
-constexpr uint32_t NBUCKETS = 10000;
+constexpr uint32_t NBUCKETS = HIST_BUCKETS;
 constexpr uint32_t EPS_CHUNK = 256;
 #ifndef KNNSJ_HIST_SPLIT
 #define KNNSJ_HIST_SPLIT 16
@@ -122,20 +122,58 @@ __global__ void eps_avg_sample_kernel(const double* __restrict__ partial, uint64
   sample_sum[g] = s;
 }
 
+// Constants of the histogram's brackets for the buckets [b_lo, b_hi).  (They
+// were computed by every thread of the histogram kernel: five double divisions
+// at 1/64 rate in each of 8000 blocks, 222 us for 100 000 points whose
+// distances take 10 us.)
+__device__ HistConst hist_const(double avg, uint32_t d, uint32_t b_lo, uint32_t b_hi, double abs_err) {
+  HistConst c;
+  c.avg = avg;
+  c.bw = __ddiv_rn(avg, NBUCKETS * 1.0);  // GPU.cu:3356
+  c.inv_bw = (float)(1.0 / c.bw);
+  c.errc = (float)(2 * d + 8) * 5.9604645e-8f;  // (2d+8) * 2^-24, relative
+  c.abs_q = (float)(abs_err / c.bw) * 1.0001f + 1e-4f;
+  c.flo = (float)b_lo;
+  c.fhi = (float)b_hi;
+  // squared-distance prefilter: a pair whose float squared distance is at
+  // least s_hi has q32 - del >= fhi (the kernel's bracket puts it above the
+  // counted range) -- q32 is within 2^-23 of sqrt(s32) / bw, and s_hi is
+  // widened by 2^-20 for its own rounding -- so it is skipped without a root
+  const double q_need = ((double)c.fhi + (double)c.abs_q) / (1.0 - (double)c.errc);
+  const double sq_bw = q_need * c.bw / ((1.0 - 1.0 / 8388608.0) * (1.0 - 1.0 / 8388608.0));
+  c.s_hi = __double2float_ru(sq_bw * sq_bw * (1.0 + 1.0 / 1048576.0));
+  return c;
+}
+
 // One warp: lane j adds the per-sample sums of the j-th of 32 contiguous
 // groups of samples in sample order, then the 32 group sums are added in
-// group order; cnt = number of terms.
+// group order; cnt = number of terms.  Then the constants of the histogram:
+// lane r those of bucket range r.
+template <typename T>
 __global__ void eps_avg_final_kernel(const double* __restrict__ sample_sum, uint64_t nthr, unsigned long long cnt,
-                                     double* __restrict__ out) {
+                                     const T* __restrict__ minmax, uint32_t d, double* __restrict__ out,
+                                     HistConst* __restrict__ hc) {
   const int lane = threadIdx.x & 31;
   const uint64_t group = (nthr + 31) / 32;
   const uint64_t g_end = min(nthr, (uint64_t)(lane + 1) * group);
   double gs = 0.0;
+#pragma unroll 8
   for (uint64_t g = (uint64_t)lane * group; g < g_end; g++) gs = __dadd_rn(gs, sample_sum[g]);
   double tot = 0.0;
   for (int j = 0; j < 32; j++) tot = __dadd_rn(tot, __shfl_sync(FULL, gs, j));
+  const double avg = __ddiv_rn(tot, (double)cnt);  // GPU.cu:3339: total/(cnt*1.0)
+  // largest |coordinate|: bounds the brackets' error from rounding double
+  // coordinates to float
+  double m = 0.0;
+  if (sizeof(T) == 8) {
+    for (uint32_t j = lane; j < 2 * d; j += 32) m = fmax(m, fabs((double)minmax[j]));
+    for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(FULL, m, off));
+    m = sqrt((double)d) * (m * (1.0 / 4194304.0));
+  }
+  if (lane < 2)
+    hc[lane] = hist_const(avg, d, lane ? HIST_FIRST : 0u, lane ? HIST_BUCKETS : HIST_FIRST, m);
   if (lane == 0) {
-    out[0] = __ddiv_rn(tot, (double)cnt);  // GPU.cu:3339: total/(cnt*1.0)
+    out[0] = avg;
     out[1] = (double)cnt;
   }
 }
@@ -149,38 +187,6 @@ __device__ __forceinline__ uint32_t exact_bucket(double rd, double avg, double b
   return b < NBUCKETS ? b : NBUCKETS;
 }
 
-// The constants of a histogram launch, from the mean distance the host has
-// read by then.  (Computed by every thread on the device, their double
-// divisions took 1/64-rate FP64 time in each of the 8000 blocks: 222 us for
-// 100 000 points, whose distances take 10 us.)
-struct HistConst {
-  double avg, bw;
-  float inv_bw, errc, abs_q, flo, fhi, s_hi;
-};
-static float float_up(double x) {
-  float f = (float)x;
-  if ((double)f < x) f = std::nextafterf(f, HUGE_VALF);
-  return f;
-}
-static HistConst hist_const(double avg, uint32_t d, uint32_t b_lo, uint32_t b_hi, double abs_err) {
-  HistConst c;
-  c.avg = avg;
-  c.bw = avg / (NBUCKETS * 1.0);  // GPU.cu:3356
-  c.inv_bw = (float)(1.0 / c.bw);
-  c.errc = (float)(2 * d + 8) * 5.9604645e-8f;  // (2d+8) * 2^-24, relative
-  c.abs_q = (float)(abs_err / c.bw) * 1.0001f + 1e-4f;
-  c.flo = (float)b_lo;
-  c.fhi = (float)b_hi;
-  // squared-distance prefilter: a pair whose float squared distance is at
-  // least s_hi has q32 - del >= fhi (the kernel's bracket puts it above the
-  // counted range) -- q32 is within 2^-23 of sqrt(s32) / bw, and s_hi is
-  // widened by 2^-20 for its own rounding -- so it is skipped without a root
-  const double q_need = ((double)c.fhi + (double)c.abs_q) / (1.0 - (double)c.errc);
-  const double sq_bw = q_need * c.bw / ((1.0 - 1.0 / 8388608.0) * (1.0 - 1.0 / 8388608.0));
-  c.s_hi = float_up(sq_bw * sq_bw * (1.0 + 1.0 / 1048576.0));
-  return c;
-}
-
 // Counts the buckets in [b_lo, b_hi) of sample blocks.  The brackets use the
 // float columns soaf; abs_err (in the constants) bounds the distance error
 // from rounding the coordinates to float (0 for float data).
@@ -188,11 +194,13 @@ template <typename T>
 __global__ void __launch_bounds__(EPS_BLOCK) eps_hist_kernel(const T* __restrict__ soa,
                                                              const float* __restrict__ soaf, uint64_t n, uint32_t d,
                                                              uint32_t offset, uint32_t* __restrict__ hist,
-                                                             uint32_t b_lo, uint32_t b_hi, const HistConst hc) {
+                                                             uint32_t b_lo, uint32_t b_hi,
+                                                             const HistConst* __restrict__ hcp) {
   extern __shared__ uint32_t sh[];  // the b_hi - b_lo counted buckets
   const uint32_t nb = b_hi - b_lo;
   for (uint32_t i = threadIdx.x; i < nb; i += blockDim.x) sh[i] = 0;
   __syncthreads();
+  const HistConst hc = *hcp;
   const double avg = hc.avg, bw = hc.bw;
   // HIST_SPLIT blocks share one sample point, each taking every
   // HIST_SPLIT-th round of candidates (integer counts: the order of the
@@ -279,7 +287,7 @@ uint32_t eps_sample_offset(uint64_t n) {
 }
 
 template <typename T>
-void launch_eps_avg(const T* soa, uint64_t n, uint32_t d, const EpsScratch& sc, cudaStream_t s) {
+void launch_eps_avg(const T* soa, const T* minmax, uint64_t n, uint32_t d, const EpsScratch& sc, cudaStream_t s) {
   const uint64_t nthr = eps_avg_threads(n);
   const uint32_t nch = eps_avg_chunks(n);
   const uint64_t work = nthr * nch;
@@ -294,29 +302,31 @@ void launch_eps_avg(const T* soa, uint64_t n, uint32_t d, const EpsScratch& sc, 
   unsigned long long cnt = 0;
   for (uint64_t g = 0; g < nthr; g++)
     if (g * 1000 < n) cnt += terms_of_sample(g, n);
-  eps_avg_final_kernel<<<1, 32, 0, s>>>(sc.sample_sum, nthr, cnt, sc.avg_out);
+  eps_avg_final_kernel<T><<<1, 32, 0, s>>>(sc.sample_sum, nthr, cnt, minmax, d, sc.avg_out, sc.hc);
   KNNSJ_CHECK_LAUNCH();
 }
 
 template <typename T>
-void launch_eps_hist(const T* soa, const float* soaf, uint64_t n, uint32_t d, const EpsScratch& sc, double avg,
-                     uint32_t b_lo, uint32_t b_hi, double abs_err, cudaStream_t s) {
+void launch_eps_hist(const T* soa, const float* soaf, uint64_t n, uint32_t d, const EpsScratch& sc, int range,
+                     cudaStream_t s) {
   const uint32_t offset = eps_sample_offset(n);
   const uint32_t blocks2 = (uint32_t)n / offset;  // GPU.cu:3440 (integer division)
-  if (blocks2 > 0 && b_hi > b_lo) {
+  const uint32_t b_lo = range ? HIST_FIRST : 0u, b_hi = range ? HIST_BUCKETS : HIST_FIRST;
+  if (blocks2 > 0) {
     // shared memory for the counted bucket range only (256 buckets on the
     // first try: a small footprint lets more blocks share an SM)
     eps_hist_kernel<T><<<blocks2 * HIST_SPLIT, EPS_BLOCK, (size_t)(b_hi - b_lo) * 4, s>>>(
-        soa, soaf, n, d, offset, sc.hist, b_lo, b_hi, hist_const(avg, d, b_lo, b_hi, abs_err));
+        soa, soaf, n, d, offset, sc.hist, b_lo, b_hi, sc.hc + range);
     KNNSJ_CHECK_LAUNCH();
   }
 }
 
-template void launch_eps_avg<float>(const float*, uint64_t, uint32_t, const EpsScratch&, cudaStream_t);
-template void launch_eps_avg<double>(const double*, uint64_t, uint32_t, const EpsScratch&, cudaStream_t);
-template void launch_eps_hist<float>(const float*, const float*, uint64_t, uint32_t, const EpsScratch&, double,
-                                     uint32_t, uint32_t, double, cudaStream_t);
-template void launch_eps_hist<double>(const double*, const float*, uint64_t, uint32_t, const EpsScratch&, double,
-                                      uint32_t, uint32_t, double, cudaStream_t);
+template void launch_eps_avg<float>(const float*, const float*, uint64_t, uint32_t, const EpsScratch&, cudaStream_t);
+template void launch_eps_avg<double>(const double*, const double*, uint64_t, uint32_t, const EpsScratch&,
+                                     cudaStream_t);
+template void launch_eps_hist<float>(const float*, const float*, uint64_t, uint32_t, const EpsScratch&, int,
+                                     cudaStream_t);
+template void launch_eps_hist<double>(const double*, const float*, uint64_t, uint32_t, const EpsScratch&, int,
+                                      cudaStream_t);
 
 }  // namespace knnsj

@@ -245,8 +245,9 @@ __global__ void cell_count_kernel(const unsigned long long* __restrict__ sk, uin
 }
 
 __global__ void dense_table_kernel(const unsigned long long* __restrict__ ckeys,
-                                   const uint32_t* __restrict__ coff, unsigned long long C,
+                                   const uint32_t* __restrict__ coff, const unsigned long long* __restrict__ dC,
                                    unsigned long long total, uint32_t* __restrict__ dstart) {
+  const unsigned long long C = *dC;
   for (unsigned long long L = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; L <= total;
        L += (unsigned long long)gridDim.x * blockDim.x) {
     unsigned long long lo = 0, hi = C;
@@ -372,6 +373,24 @@ __global__ void cell_scatter_atomic_kernel(const T* __restrict__ src, const uint
   }
 }
 
+// Marks every point's cell in a bitmap and counts the cells marked first.
+template <typename T>
+__global__ void cell_mark_kernel(const T* __restrict__ soa, uint64_t n, const GridGeom<T> g,
+                                 uint32_t* __restrict__ bitmap, unsigned long long* __restrict__ count) {
+  uint32_t fresh = 0;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    // (never past the bitmap, whatever the rounding at the grid's far edge)
+    const unsigned long long lin = min(cell_of(soa, n, i, g), g.total_cells - 1ull);
+    const uint32_t bit = 1u << (lin & 31u);
+    uint32_t* w = &bitmap[lin >> 5];
+    // (a stale 0 only costs an atomic)
+    if (!(*(volatile uint32_t*)w & bit) && !(atomicOr(w, bit) & bit)) fresh++;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) fresh += __shfl_xor_sync(FULL, fresh, off);
+  if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(count, (unsigned long long)fresh);
+}
+
 unsigned grid_blocks(uint64_t n, int threads = 256) {
   uint64_t b = (n + threads - 1) / threads;
   if (b > 152ull * 64) b = 152ull * 64;
@@ -431,9 +450,17 @@ void launch_compact_cells(const unsigned long long* skeys, uint64_t n, uint32_t*
   KNNSJ_CHECK_LAUNCH();
 }
 
-void launch_dense_table(const unsigned long long* ckeys, const uint32_t* coff, unsigned long long C,
+void launch_dense_table(const unsigned long long* ckeys, const uint32_t* coff, const unsigned long long* d_C,
                         unsigned long long total_cells, uint32_t* dstart, cudaStream_t s) {
-  dense_table_kernel<<<grid_blocks(total_cells + 1), 256, 0, s>>>(ckeys, coff, C, total_cells, dstart);
+  dense_table_kernel<<<grid_blocks(total_cells + 1), 256, 0, s>>>(ckeys, coff, d_C, total_cells, dstart);
+  KNNSJ_CHECK_LAUNCH();
+}
+
+template <typename T>
+void launch_count_cells(const T* soa, uint64_t n, const GridGeom<T>& g, uint32_t* bitmap, unsigned long long* d_C,
+                        cudaStream_t s) {
+  launch_zero_words(bitmap, (size_t)((g.total_cells + 31) / 32) * 4, s);
+  cell_mark_kernel<T><<<grid_blocks(n), 256, 0, s>>>(soa, n, g, bitmap, d_C);
   KNNSJ_CHECK_LAUNCH();
 }
 
@@ -466,6 +493,10 @@ template void launch_cell_ids<float>(const float*, uint64_t, const GridGeom<floa
                                      uint32_t*, cudaStream_t);
 template void launch_cell_ids<double>(const double*, uint64_t, const GridGeom<double>&, unsigned long long*,
                                       uint32_t*, cudaStream_t);
+template void launch_count_cells<float>(const float*, uint64_t, const GridGeom<float>&, uint32_t*,
+                                        unsigned long long*, cudaStream_t);
+template void launch_count_cells<double>(const double*, uint64_t, const GridGeom<double>&, uint32_t*,
+                                         unsigned long long*, cudaStream_t);
 template void launch_morton_keys<float>(const float*, uint64_t, const GridGeom<float>&, int, unsigned long long*,
                                         uint32_t*, cudaStream_t);
 template void launch_morton_keys<double>(const double*, uint64_t, const GridGeom<double>&, int,

@@ -7,6 +7,7 @@
 //  * minmax: per-dimension minimum and maximum of the indexed dimensions, the
 //    first half of generateNDGridDimensions (main.cu:2425-2460).
 
+#include <algorithm>
 #include <cfloat>
 
 #include "exact_sqrt.cuh"
@@ -16,21 +17,33 @@ namespace knnsj {
 
 namespace {
 
+struct DimOrder {
+  uint16_t p[MAX_D];
+};
+
 template <typename T>
 __global__ void transpose_reorder_kernel(const T* __restrict__ aos, T* __restrict__ soa, float* __restrict__ soaf,
-                                         uint64_t n, uint32_t d, const uint32_t* __restrict__ perm,
+                                         uint64_t n, uint32_t d, const DimOrder perm,
                                          uint32_t* __restrict__ nonfinite) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   bool bad = false;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     for (uint32_t j = 0; j < d; j++) {
-      const T v = aos[i * d + perm[j]];
+      const T v = aos[i * d + perm.p[j]];
       bad |= !isfinite(v);
       soa[(uint64_t)j * n + i] = v;
       if (soaf) soaf[(uint64_t)j * n + i] = (float)v;
     }
   }
   if (__any_sync(FULL, bad) && (threadIdx.x & 31) == 0) atomicOr(nonfinite, 1u);
+}
+
+template <typename T>
+__global__ void gather_rows_kernel(const T* __restrict__ aos, uint64_t count, uint64_t step, uint32_t d,
+                                   T* __restrict__ out) {
+  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < count * d;
+       e += (uint64_t)gridDim.x * blockDim.x)
+    out[e] = aos[e / d * step * d + e % d];
 }
 
 template <typename T>
@@ -171,11 +184,20 @@ template void launch_checksum<double>(const double*, uint64_t, double*, double*,
 constexpr uint32_t MINMAX_BLOCKS = 1024;
 
 template <typename T>
-void launch_transpose_reorder(const T* aos, T* soa, float* soaf, uint64_t n, uint32_t d, const uint32_t* d_perm,
+void launch_transpose_reorder(const T* aos, T* soa, float* soaf, uint64_t n, uint32_t d, const uint32_t* perm,
                               cudaStream_t s, uint32_t* d_nonfinite) {
+  DimOrder order{};
+  for (uint32_t j = 0; j < d; j++) order.p[j] = (uint16_t)perm[j];
   uint64_t blocks = (n + 255) / 256;
   if (blocks > 152ull * 32) blocks = 152ull * 32;
-  transpose_reorder_kernel<T><<<(unsigned)blocks, 256, 0, s>>>(aos, soa, soaf, n, d, d_perm, d_nonfinite);
+  transpose_reorder_kernel<T><<<(unsigned)blocks, 256, 0, s>>>(aos, soa, soaf, n, d, order, d_nonfinite);
+  KNNSJ_CHECK_LAUNCH();
+}
+
+template <typename T>
+void launch_gather_rows(const T* aos, uint64_t count, uint64_t step, uint32_t d, T* out, cudaStream_t s) {
+  const uint64_t blocks = std::min<uint64_t>((count * d + 255) / 256, 152ull * 8);
+  gather_rows_kernel<T><<<(unsigned)std::max<uint64_t>(blocks, 1), 256, 0, s>>>(aos, count, step, d, out);
   KNNSJ_CHECK_LAUNCH();
 }
 
@@ -194,6 +216,8 @@ template void launch_transpose_reorder<float>(const float*, float*, float*, uint
                                               cudaStream_t, uint32_t*);
 template void launch_transpose_reorder<double>(const double*, double*, float*, uint64_t, uint32_t,
                                                const uint32_t*, cudaStream_t, uint32_t*);
+template void launch_gather_rows<float>(const float*, uint64_t, uint64_t, uint32_t, float*, cudaStream_t);
+template void launch_gather_rows<double>(const double*, uint64_t, uint64_t, uint32_t, double*, cudaStream_t);
 template void launch_minmax<float>(const float*, uint64_t, uint32_t, float*, float*, cudaStream_t);
 template void launch_minmax<double>(const double*, uint64_t, uint32_t, double*, double*, cudaStream_t);
 

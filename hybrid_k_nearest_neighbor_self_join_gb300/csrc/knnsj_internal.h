@@ -76,29 +76,42 @@ struct DeviceGrid {
 
 // ---- kernel launchers (k_*.cu) -------------------------------------------
 template <typename T>
-// (soaf, optional: the columns rounded to float as well)
-void launch_transpose_reorder(const T* aos, T* soa, float* soaf, uint64_t n, uint32_t d, const uint32_t* d_perm,
+// perm (host): input dimension of each column; soaf (optional): the columns
+// rounded to float as well.
+void launch_transpose_reorder(const T* aos, T* soa, float* soaf, uint64_t n, uint32_t d, const uint32_t* perm,
                               cudaStream_t s, uint32_t* d_nonfinite);
+// Every `step`-th row (rows 0, step, ...; count of them), densely packed.
+template <typename T>
+void launch_gather_rows(const T* aos, uint64_t count, uint64_t step, uint32_t d, T* out, cudaStream_t s);
 template <typename T>
 void launch_minmax(const T* soa, uint64_t n, uint32_t di, T* d_minmax /*2*di*/, T* scratch /*1024*2*di*/,
                    cudaStream_t s);
 
+// Constants of the distance histogram (k_eps.cu) for a range of buckets.
+struct HistConst {
+  double avg, bw;
+  float inv_bw, errc, abs_q, flo, fhi, s_hi;
+};
+constexpr uint32_t HIST_FIRST = 256;  // buckets [0, HIST_FIRST) are counted first, the rest if need be
+constexpr uint32_t HIST_BUCKETS = 10000;
 struct EpsScratch {
   double* partial = nullptr;     // [eps_avg_threads * eps_avg_chunks]
   double* sample_sum = nullptr;  // [eps_avg_threads]
   double* avg_out = nullptr;     // [2]: mean distance, pair count
-  uint32_t* hist = nullptr;      // [10000]
+  uint32_t* hist = nullptr;      // [HIST_BUCKETS]
+  HistConst* hc = nullptr;       // [2]: constants of the two bucket ranges
 };
 uint64_t eps_avg_threads(uint64_t n);
 uint32_t eps_avg_chunks(uint64_t n);
 uint32_t eps_sample_offset(uint64_t n);
 template <typename T>
-void launch_eps_avg(const T* soa, uint64_t n, uint32_t d, const EpsScratch& sc, cudaStream_t s);
+// (minmax: the columns' extremes, for the histogram's constants)
+void launch_eps_avg(const T* soa, const T* minmax, uint64_t n, uint32_t d, const EpsScratch& sc, cudaStream_t s);
 template <typename T>
-// avg: the sampled mean distance (*avg_out); soaf: the columns rounded to
-// float (float data: the columns themselves).
-void launch_eps_hist(const T* soa, const float* soaf, uint64_t n, uint32_t d, const EpsScratch& sc, double avg,
-                     uint32_t b_lo, uint32_t b_hi, double abs_err, cudaStream_t s);
+// soaf: the columns rounded to float (float data: the columns themselves);
+// range 0 or 1: which of the two bucket ranges is counted.
+void launch_eps_hist(const T* soa, const float* soaf, uint64_t n, uint32_t d, const EpsScratch& sc, int range,
+                     cudaStream_t s);
 // Sum of squared result distances (the reference's verification figure,
 // GPU.cu:3690-3693) in a fixed order; result in *d_out.
 template <typename T>
@@ -129,8 +142,12 @@ int radix_sort_pairs(GridScratch& sc, uint64_t n, int bits, cudaStream_t s);
 void launch_compact_cells(const unsigned long long* skeys, uint64_t n, uint32_t* flags,
                           uint32_t* pos, uint32_t* scan_tmp, unsigned long long* ckeys,
                           uint32_t* coff, unsigned long long* d_C, cudaStream_t s);
-void launch_dense_table(const unsigned long long* ckeys, const uint32_t* coff,
-                        unsigned long long C, unsigned long long total_cells, uint32_t* dstart,
+void launch_dense_table(const unsigned long long* ckeys, const uint32_t* coff, const unsigned long long* d_C,
+                        unsigned long long total_cells, uint32_t* dstart, cudaStream_t s);
+// Number of cells that hold a point into *d_C, by a bitmap of the grid's cells
+// (total_cells bits, rounded up to words).
+template <typename T>
+void launch_count_cells(const T* soa, uint64_t n, const GridGeom<T>& g, uint32_t* bitmap, unsigned long long* d_C,
                         cudaStream_t s);
 // Morton (Z-order) codes of the cells of points given in cell-ordered
 // columns ps (keys) and their positions (vals), `bits` bits per dimension.
@@ -246,7 +263,7 @@ void launch_brute(const SearchLaunch<T>& a, cudaStream_t s);
 // its search is done, and the rows that later passes finish are written into
 // the host buffers by a kernel at the end, after every chunk copy.
 constexpr int MAX_ROW_CHUNKS = 32;
-constexpr size_t MAIL_BYTES = 4096;  // mailbox: reads in the first half, writes in the second
+constexpr size_t MAIL_BYTES = 16384;  // mailbox: reads in the first half, writes in the second
 struct RowStream {
   void* ids_host = nullptr;  // the host buffers
   void* d_host = nullptr;
@@ -331,10 +348,12 @@ struct Workspace {
   cudaEvent_t ev[8] = {};
   cudaStream_t copy_stream = nullptr;    // streamed rows: device-to-host copies
   cudaEvent_t chunk_ev[MAX_ROW_CHUNKS + 1] = {};
-  // While rows stream out, the copy engines are busy for tens of ms: the
-  // join's small reads and writes of host memory then go through the mailbox
-  // (mapped pinned memory that kernels read and write), device copies run on
-  // the SMs, and none of them queues behind the row copies.
+  // The join's small reads of device memory go through the mailbox (mapped
+  // pinned memory that a kernel writes): one kernel and one synchronisation
+  // for several pieces, where each copy into pageable memory is staged and
+  // waited for by itself.  While rows stream out, the copy engines are busy
+  // for tens of ms: small writes then take the mailbox too, device copies run
+  // on the SMs (`mail` set), and none of them queues behind the row copies.
   void* mail_host = nullptr;
   void* mail_dev = nullptr;
   bool mail = false;
@@ -342,7 +361,8 @@ struct Workspace {
   void* h_pinned = nullptr;
   size_t h_pinned_bytes = 0;
   void ensure_stream();
-  void ensure_copy_stream();  // and the mailbox
+  void ensure_copy_stream();
+  void ensure_mail();
   void* pinned(size_t need);
   void pinned_release();
   void release_all();
