@@ -137,11 +137,20 @@ __global__ void checksum_kernel(const T* __restrict__ v, uint64_t count, double*
   }
 }
 
-__global__ void checksum_final_kernel(const double* __restrict__ part, unsigned nb, double* __restrict__ out) {
-  if (threadIdx.x != 0) return;
-  double t = 0.0;
-  for (unsigned b = 0; b < nb; b++) t += part[b];
-  *out = t;
+// One block: the block partials in a fixed tree.  (One thread adding the 1024
+// of them in a row took 61 us.)
+__global__ void __launch_bounds__(CHECKSUM_BLOCKS) checksum_final_kernel(const double* __restrict__ part,
+                                                                        double* __restrict__ out) {
+  __shared__ double ws[32];
+  double s = part[threadIdx.x];
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL, s, off);
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = ws[threadIdx.x];
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(FULL, s, off);
+    if (threadIdx.x == 0) *out = s;
+  }
 }
 
 // Sum of n doubles in a fixed order: grid-stride partial sums per thread,
@@ -167,7 +176,7 @@ __global__ void sum_f64_kernel(const double* __restrict__ v, uint64_t count, dou
 void launch_sum_f64(const double* v, uint64_t count, double* d_partial, double* d_out, cudaStream_t s) {
   sum_f64_kernel<<<CHECKSUM_BLOCKS, 256, 0, s>>>(v, count, d_partial);
   KNNSJ_CHECK_LAUNCH();
-  checksum_final_kernel<<<1, 32, 0, s>>>(d_partial, CHECKSUM_BLOCKS, d_out);
+  checksum_final_kernel<<<1, CHECKSUM_BLOCKS, 0, s>>>(d_partial, d_out);
   KNNSJ_CHECK_LAUNCH();
 }
 
@@ -175,7 +184,7 @@ template <typename T>
 void launch_checksum(const T* dists, uint64_t count, double* d_partial, double* d_out, cudaStream_t s) {
   checksum_kernel<T><<<CHECKSUM_BLOCKS, 256, 0, s>>>(dists, count, d_partial);
   KNNSJ_CHECK_LAUNCH();
-  checksum_final_kernel<<<1, 32, 0, s>>>(d_partial, CHECKSUM_BLOCKS, d_out);
+  checksum_final_kernel<<<1, CHECKSUM_BLOCKS, 0, s>>>(d_partial, d_out);
   KNNSJ_CHECK_LAUNCH();
 }
 template void launch_checksum<float>(const float*, uint64_t, double*, double*, cudaStream_t);
