@@ -394,10 +394,10 @@ static void build_grid(Workspace& w, const JoinConfig& cfg, uint64_t n, uint32_t
   unsigned long long* ckeys = (unsigned long long*)w.ckeys.get(n * 8);
   uint32_t* coff = (uint32_t*)w.coff.get((n + 1) * 4);
   launch_compact_cells(skeys, n, flags, pos, sc.scan_tmp, ckeys, coff, d_C, s);
-  // (the box tree keeps its columns in the same buffers, at its own stride)
+  // (the box tree keeps its points in the same buffers, in whole leaves)
   T* ps = (T*)w.ps.get(tree_stride(n) * d * sizeof(T));
   float* psf = sizeof(T) == 8 ? (float*)w.psf.get(tree_stride(n) * d * sizeof(float)) : nullptr;
-  uint32_t* pid = (uint32_t*)w.pid.get(n * 4);
+  uint32_t* pid = (uint32_t*)w.pid.get(tree_stride(n) * 4);
   dev_copy(w, pid, sids, n * 4, s);
   launch_gather_sorted<T>(xs, n, d, sids, ps, psf, s);
   out->geom = g;
@@ -956,11 +956,10 @@ static void run_tree(Workspace& w, const Prepared<T>& P, uint64_t n, uint32_t d,
                            cudaStream_t s) {
   BoxTree<T> t;
   tree_shape(n, d, t.count, t.offset, &t.levels, &t.nodes);
-  t.ld = tree_stride(n);
   t.dims = std::min(d, TREE_DIMS);
-  t.ps = (T*)w.ps.get(t.ld * d * sizeof(T));
-  t.psf = sizeof(T) == 8 ? (float*)w.psf.get(t.ld * d * sizeof(float)) : nullptr;
-  t.id = (uint32_t*)w.pid.get(n * 4);
+  t.ps = (T*)w.ps.get(tree_stride(n) * d * sizeof(T));
+  t.psf = sizeof(T) == 8 ? (float*)w.psf.get(tree_stride(n) * d * sizeof(float)) : nullptr;
+  t.id = (uint32_t*)w.pid.get(tree_stride(n) * 4);
   t.box = (float*)w.tree_box.get((size_t)2 * t.dims * t.nodes * 4);
   TreeScratch sc;
   sc.sort.keys[0] = (unsigned long long*)w.keys0.get(n * 8);

@@ -22,7 +22,7 @@ namespace {
 
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ITEMS = 8;                       // rounds of 32 keys per warp
+constexpr int RS_ITEMS = 16;                      // rounds of 32 keys per warp
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;    // keys per block tile
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
@@ -43,8 +43,23 @@ __global__ void cell_id_kernel(const T* __restrict__ soa, uint64_t n, const Grid
   }
 }
 
-__global__ void radix_hist_kernel(const unsigned long long* __restrict__ keys, uint64_t n, int shift,
-                                  uint32_t ntiles, uint32_t* __restrict__ hist) {
+// A radix pass is three launches: the digit counts of each tile of 4096 keys,
+// per digit the running sums over the tiles (one block per digit), and the
+// scatter, which sorts its tile by digit in shared memory first, so that a
+// digit's keys leave in one run.  (Scattering straight from registers wrote
+// single keys; 116 us per pass of 10 M pairs, 28 us of scan and five launches.)
+//
+// `limit` (optional): the largest key; a pass whose digits are all zero is
+// skipped by every kernel, and the pairs stay where they are.
+__device__ __forceinline__ bool pass_empty(const unsigned long long* limit, int shift) {
+  return limit && (*limit >> shift) == 0;
+}
+
+__global__ void __launch_bounds__(RS_THREADS) radix_hist_kernel(const unsigned long long* __restrict__ keys, uint64_t n,
+                                                                int shift, uint32_t ntiles,
+                                                                uint32_t* __restrict__ hist,
+                                                                const unsigned long long* __restrict__ limit) {
+  if (pass_empty(limit, shift)) return;
   __shared__ uint32_t cnt[256];
   cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -58,61 +73,132 @@ __global__ void radix_hist_kernel(const unsigned long long* __restrict__ keys, u
   hist[(uint64_t)threadIdx.x * ntiles + blockIdx.x] = cnt[threadIdx.x];
 }
 
-// Stable scatter: warp w owns keys [tile + w*256, tile + w*256 + 256) and
-// visits them in order, 32 at a time; equal digits within a round are ranked
-// by lane, rounds by order, warps by index, tiles by the scanned histogram.
-__global__ void radix_scatter_kernel(const unsigned long long* __restrict__ kin,
-                                     const uint32_t* __restrict__ vin, unsigned long long* __restrict__ kout,
-                                     uint32_t* __restrict__ vout, uint64_t n, int shift, uint32_t ntiles,
-                                     const uint32_t* __restrict__ offs) {
-  __shared__ uint32_t wc[RS_WARPS][256];
+// Exclusive sum over a block's RS_THREADS values; total in every thread.
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* ws, uint32_t& total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) (&wc[0][0])[i] = 0;
+  uint32_t incl = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t t = __shfl_up_sync(FULL, incl, off);
+    if (lane >= off) incl += t;
+  }
+  __syncthreads();  // (ws may still be read from the last call)
+  if (lane == 31) ws[w] = incl;
   __syncthreads();
-  const uint64_t wbase = (uint64_t)blockIdx.x * RS_TILE + (uint64_t)w * (RS_ITEMS * 32);
+  uint32_t before = 0;
+  total = 0;
+#pragma unroll
+  for (int k = 0; k < RS_WARPS; k++) {
+    if (k < w) before += ws[k];
+    total += ws[k];
+  }
+  return before + incl - v;
+}
+
+// Block d: exclusive running sums of digit d's counts over the tiles, in
+// place, and their total.
+__global__ void __launch_bounds__(RS_THREADS) radix_rows_kernel(uint32_t* __restrict__ hist, uint32_t ntiles, int shift,
+                                                                uint32_t* __restrict__ total,
+                                                                const unsigned long long* __restrict__ limit) {
+  if (pass_empty(limit, shift)) return;
+  __shared__ uint32_t ws[RS_WARPS];
+  uint32_t* row = hist + (uint64_t)blockIdx.x * ntiles;
+  uint32_t carry = 0;
+  for (uint32_t t0 = 0; t0 < ntiles; t0 += RS_THREADS * 4) {
+    uint32_t x[4], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t t = t0 + threadIdx.x * 4 + j;
+      x[j] = t < ntiles ? row[t] : 0u;
+      sum += x[j];
+    }
+    uint32_t all;
+    uint32_t run = carry + block_exclusive(sum, ws, all);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t t = t0 + threadIdx.x * 4 + j;
+      if (t < ntiles) row[t] = run;
+      run += x[j];
+    }
+    carry += all;
+  }
+  if (threadIdx.x == 0) total[blockIdx.x] = carry;
+}
+
+// Stable scatter: warp w owns keys [tile + 512 w, tile + 512 w + 512) and
+// visits them in order, 32 at a time; equal digits within a round are ranked
+// by lane, rounds by order, warps by index, tiles by the running sums.
+constexpr int RS_SMEM = RS_TILE * 12 + RS_WARPS * 256 * 4 + 256 * 4;
+__global__ void __launch_bounds__(RS_THREADS) radix_scatter_kernel(
+    const unsigned long long* __restrict__ kin, const uint32_t* __restrict__ vin,
+    unsigned long long* __restrict__ kout, uint32_t* __restrict__ vout, uint64_t n, int shift, uint32_t ntiles,
+    const uint32_t* __restrict__ rows, const uint32_t* __restrict__ total,
+    const unsigned long long* __restrict__ limit) {
+  if (pass_empty(limit, shift)) return;
+  extern __shared__ __align__(16) unsigned char rs_smem[];
+  unsigned long long* sk = reinterpret_cast<unsigned long long*>(rs_smem);  // [RS_TILE]
+  uint32_t* sv = reinterpret_cast<uint32_t*>(sk + RS_TILE);                 // [RS_TILE]
+  uint32_t* wc = sv + RS_TILE;                                              // [RS_WARPS][256]
+  uint32_t* gb = wc + RS_WARPS * 256;                                       // [256]: global less local position
+  __shared__ uint32_t ws[RS_WARPS];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) wc[i] = 0;
+  __syncthreads();
+  const uint64_t base = (uint64_t)blockIdx.x * RS_TILE;
+  const uint64_t wbase = base + (uint64_t)w * (RS_ITEMS * 32);
   unsigned long long k[RS_ITEMS];
   uint32_t v[RS_ITEMS];
-  uint32_t dg[RS_ITEMS];
+  uint32_t at[RS_ITEMS];  // rank within the warp's keys of this digit
 #pragma unroll
   for (int r = 0; r < RS_ITEMS; r++) {
     const uint64_t idx = wbase + (uint64_t)r * 32 + lane;
-    if (idx < n) {
-      k[r] = kin[idx];
-      v[r] = vin[idx];
-      dg[r] = (uint32_t)((k[r] >> shift) & 0xff);
-    } else {
-      k[r] = 0;
-      v[r] = 0;
-      dg[r] = 256;
-    }
-    const unsigned peers = __match_any_sync(FULL, dg[r]);
-    const int leader = __ffs(peers) - 1;
-    if (lane == leader && dg[r] < 256) wc[w][dg[r]] += __popc(peers);
+    k[r] = idx < n ? kin[idx] : 0ull;
+    v[r] = idx < n ? vin[idx] : 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < RS_ITEMS; r++) {
+    const bool live = wbase + (uint64_t)r * 32 + lane < n;
+    const uint32_t dg = live ? (uint32_t)((k[r] >> shift) & 0xff) : 256u;
+    const unsigned peers = __match_any_sync(FULL, dg);
+    const uint32_t before = live ? wc[w * 256 + dg] : 0u;
     __syncwarp();
+    if (live && lane == __ffs(peers) - 1) wc[w * 256 + dg] = before + __popc(peers);
+    __syncwarp();
+    at[r] = before + __popc(peers & lanemask_lt());
   }
   __syncthreads();
   {
     const int digit = threadIdx.x;  // RS_THREADS == 256
-    uint32_t run = offs[(uint64_t)digit * ntiles + blockIdx.x];
+    uint32_t here = 0;
     for (int ww = 0; ww < RS_WARPS; ww++) {
-      const uint32_t c = wc[ww][digit];
-      wc[ww][digit] = run;
-      run += c;
+      const uint32_t c = wc[ww * 256 + digit];
+      wc[ww * 256 + digit] = here;
+      here += c;
     }
+    uint32_t all;
+    const uint32_t start = block_exclusive(here, ws, all);
+    const uint32_t global = block_exclusive(total[digit], ws, all) + rows[(uint64_t)digit * ntiles + blockIdx.x];
+    for (int ww = 0; ww < RS_WARPS; ww++) wc[ww * 256 + digit] += start;
+    gb[digit] = global - start;
   }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < RS_ITEMS; r++) {
-    const unsigned peers = __match_any_sync(FULL, dg[r]);
-    const int leader = __ffs(peers) - 1;
-    if (dg[r] < 256) {
-      const uint32_t dst = wc[w][dg[r]] + __popc(peers & lanemask_lt());
-      kout[dst] = k[r];
-      vout[dst] = v[r];
+    if (wbase + (uint64_t)r * 32 + lane < n) {
+      const uint32_t dg = (uint32_t)((k[r] >> shift) & 0xff);
+      const uint32_t lp = wc[w * 256 + dg] + at[r];
+      sk[lp] = k[r];
+      sv[lp] = v[r];
     }
-    __syncwarp();
-    if (lane == leader && dg[r] < 256) wc[w][dg[r]] += __popc(peers);
-    __syncwarp();
+  }
+  __syncthreads();
+  const uint32_t count = (uint32_t)min((unsigned long long)RS_TILE, (unsigned long long)(n - base));
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < count; i += RS_THREADS) {
+    const unsigned long long key = sk[i];
+    const uint32_t dst = gb[(key >> shift) & 0xff] + i;
+    kout[dst] = key;
+    vout[dst] = sv[i];
   }
 }
 
@@ -400,7 +486,8 @@ unsigned grid_blocks(uint64_t n, int threads = 256) {
 
 }  // namespace
 
-size_t radix_hist_elems(uint64_t n) { return (size_t)256 * ((n + RS_TILE - 1) / RS_TILE); }
+// (tile counts of every digit, then the digits' totals)
+size_t radix_hist_elems(uint64_t n) { return (size_t)256 * ((n + RS_TILE - 1) / RS_TILE) + 256; }
 
 size_t scan_tmp_elems(size_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE + 1; }
 
@@ -422,16 +509,19 @@ void launch_cell_ids(const T* soa, uint64_t n, const GridGeom<T>& g, unsigned lo
   KNNSJ_CHECK_LAUNCH();
 }
 
-int radix_sort_pairs(GridScratch& sc, uint64_t n, int bits, cudaStream_t s) {
+int radix_sort_pairs(GridScratch& sc, uint64_t n, int bits, cudaStream_t s, const unsigned long long* limit) {
   int cur = 0;
   const uint32_t ntiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
-  const size_t nh = (size_t)256 * ntiles;
+  uint32_t* total = sc.hist + (size_t)256 * ntiles;
+  KNNSJ_CUDA(cudaFuncSetAttribute(radix_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM));
   for (int shift = 0; shift < bits; shift += 8) {
-    radix_hist_kernel<<<ntiles, RS_THREADS, 0, s>>>(sc.keys[cur], n, shift, ntiles, sc.hist);
+    radix_hist_kernel<<<ntiles, RS_THREADS, 0, s>>>(sc.keys[cur], n, shift, ntiles, sc.hist, limit);
     KNNSJ_CHECK_LAUNCH();
-    scan_exclusive_u32(sc.hist, sc.hist, nh, sc.scan_tmp, s);
-    radix_scatter_kernel<<<ntiles, RS_THREADS, 0, s>>>(sc.keys[cur], sc.vals[cur], sc.keys[cur ^ 1],
-                                                       sc.vals[cur ^ 1], n, shift, ntiles, sc.hist);
+    radix_rows_kernel<<<256, RS_THREADS, 0, s>>>(sc.hist, ntiles, shift, total, limit);
+    KNNSJ_CHECK_LAUNCH();
+    radix_scatter_kernel<<<ntiles, RS_THREADS, RS_SMEM, s>>>(sc.keys[cur], sc.vals[cur], sc.keys[cur ^ 1],
+                                                             sc.vals[cur ^ 1], n, shift, ntiles, sc.hist, total,
+                                                             limit);
     KNNSJ_CHECK_LAUNCH();
     cur ^= 1;
   }

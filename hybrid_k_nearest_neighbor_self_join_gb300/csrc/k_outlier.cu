@@ -62,17 +62,32 @@ __global__ void total_keys_kernel(const T* __restrict__ total, uint64_t n, unsig
 }
 
 __global__ void degree_keys_kernel(const unsigned long long* __restrict__ indeg, uint64_t n,
-                                   unsigned long long* __restrict__ keys, uint32_t* __restrict__ vals) {
+                                   unsigned long long* __restrict__ keys, uint32_t* __restrict__ vals,
+                                   unsigned long long* __restrict__ largest) {
+  unsigned long long mx = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    keys[i] = indeg[i];
+    const unsigned long long v = indeg[i];
+    keys[i] = v;
     vals[i] = (uint32_t)i;
+    mx = max(mx, v);
   }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, off));
+  if ((threadIdx.x & 31) == 0 && mx) atomicMax(largest, mx);
 }
 
-template <typename R>
-__global__ void rank_scatter_kernel(const uint32_t* __restrict__ sorted_ids, uint64_t n, R* __restrict__ rank) {
+// Ranks from the sort that stopped after the highest digit of *largest.
+__global__ void degree_rank_kernel(const uint32_t* __restrict__ ids0, const uint32_t* __restrict__ ids1,
+                                   const unsigned long long* __restrict__ largest, uint64_t n,
+                                   uint32_t* __restrict__ rank) {
+  const uint32_t* ids = radix_passes(*largest) & 1 ? ids1 : ids0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    rank[sorted_ids[i]] = (R)i;
+    rank[ids[i]] = (uint32_t)i;
+}
+
+__global__ void rank_scatter_kernel(const uint32_t* __restrict__ sorted_ids, uint64_t n, int32_t* __restrict__ rank) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    rank[sorted_ids[i]] = (int32_t)i;
 }
 
 unsigned blocks_for(uint64_t n) {
@@ -107,17 +122,21 @@ void outlier_scores_device(Workspace& w, const int32_t* ids, const T* dists, uin
   KNNSJ_CHECK_LAUNCH();
   total_keys_kernel<T><<<blocks_for(n), 256, 0, s>>>(total, n, sc.keys[0], sc.vals[0]);
   KNNSJ_CHECK_LAUNCH();
-  int cur = radix_sort_pairs(sc, n, (int)(8 * sizeof(T)), s);
-  rank_scatter_kernel<int32_t><<<blocks_for(n), 256, 0, s>>>(sc.vals[cur], n, dist_rank);
+  const int cur = radix_sort_pairs(sc, n, (int)(8 * sizeof(T)), s);
+  rank_scatter_kernel<<<blocks_for(n), 256, 0, s>>>(sc.vals[cur], n, dist_rank);
   KNNSJ_CHECK_LAUNCH();
   // criterion 2: in-degrees and the order of increasing in-degree
   KNNSJ_CUDA(cudaMemsetAsync(indeg, 0, n * sizeof(unsigned long long), s));
   in_degree_kernel<<<blocks_for(n * K), 256, 0, s>>>(ids, n * K, n, indeg);
   KNNSJ_CHECK_LAUNCH();
-  degree_keys_kernel<<<blocks_for(n), 256, 0, s>>>(indeg, n, sc.keys[0], sc.vals[0]);
+  // (in-degrees rarely need more than one or two digits of the n K they could
+  // reach: the sort's further passes are skipped on the device)
+  unsigned long long* largest = (unsigned long long*)w.eps_sample.get(sizeof(unsigned long long));
+  KNNSJ_CUDA(cudaMemsetAsync(largest, 0, sizeof(*largest), s));
+  degree_keys_kernel<<<blocks_for(n), 256, 0, s>>>(indeg, n, sc.keys[0], sc.vals[0], largest);
   KNNSJ_CHECK_LAUNCH();
-  cur = radix_sort_pairs(sc, n, std::max(bits_of(n * (unsigned long long)K), 1), s);
-  rank_scatter_kernel<uint32_t><<<blocks_for(n), 256, 0, s>>>(sc.vals[cur], n, degree_rank);
+  radix_sort_pairs(sc, n, std::max(bits_of(n * (unsigned long long)K), 1), s, largest);
+  degree_rank_kernel<<<blocks_for(n), 256, 0, s>>>(sc.vals[0], sc.vals[1], largest, n, degree_rank);
   KNNSJ_CHECK_LAUNCH();
 }
 

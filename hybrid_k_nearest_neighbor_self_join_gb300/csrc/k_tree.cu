@@ -158,9 +158,9 @@ template <typename T>
 __global__ void __launch_bounds__(REFINE_THREADS) tree_refine_kernel(const T* __restrict__ xs, uint64_t n, uint32_t d,
                                                                      uint32_t rd, const uint32_t* __restrict__ ids,
                                                                      T* __restrict__ ps, float* __restrict__ psf,
-                                                                     uint32_t* __restrict__ tid, uint64_t ld,
-                                                                     float* __restrict__ box, uint32_t nodes,
-                                                                     uint32_t bd, uint32_t leaves, uint32_t off1) {
+                                                                     uint32_t* __restrict__ tid,
+                                                                     float* __restrict__ box, uint32_t bd,
+                                                                     uint32_t leaves, uint32_t off1) {
   extern __shared__ float co[];  // [rd][BLOCK_PTS]
   __shared__ unsigned long long key[BLOCK_PTS];
   __shared__ float var[16][REFINE_DIMS];
@@ -242,15 +242,16 @@ __global__ void __launch_bounds__(REFINE_THREADS) tree_refine_kernel(const T* __
   uint32_t* hib = lob + TREE_DIMS * 32;
   for (int h = 0; h < 2; h++) {
     const uint32_t leaf = warp + h * WARPS;
-    const uint64_t pos = base + leaf * 32 + lane;
+    const uint64_t node = (uint64_t)blockIdx.x * 32 + leaf;
     const bool live = leaf * 32 + lane < cnt;
-    const uint32_t id = live ? ids[base + loc[h]] : 0u;
-    if (live) tid[pos] = id;
+    const bool there = node < leaves;
+    const uint32_t id = live ? ids[base + loc[h]] : 0xffffffffu;
+    if (there) tid[node * 32 + lane] = id;
     for (uint32_t l = 0; l < d; l++) {
-      const T v = live ? xs[(uint64_t)l * n + id] : (T)0;
-      if (live) {
-        ps[(uint64_t)l * ld + pos] = v;
-        if (psf) psf[(uint64_t)l * ld + pos] = (float)v;
+      const T v = live ? xs[(uint64_t)l * n + id] : (T)INFINITY;
+      if (there) {
+        ps[(node * d + l) * 32 + lane] = v;
+        if (psf) psf[(node * d + l) * 32 + lane] = (float)v;
       }
       if (l < bd) {
         const uint32_t lo = __reduce_min_sync(FULL, live ? float_order(box_down(v)) : 0xffffffffu);
@@ -258,10 +259,10 @@ __global__ void __launch_bounds__(REFINE_THREADS) tree_refine_kernel(const T* __
         if (lane == 0) {
           lob[l * 32 + leaf] = lo;
           hib[l * 32 + leaf] = hi;
-          const uint32_t node = blockIdx.x * 32 + leaf;
-          if (node < leaves) {
-            box[(uint64_t)(2 * l) * nodes + node] = order_float(lo);
-            box[(uint64_t)(2 * l + 1) * nodes + node] = order_float(hi);
+          if (there) {
+            float* b = box + ((uint64_t)blockIdx.x * 2 * bd + 2 * l) * 32 + leaf;
+            b[0] = order_float(lo);
+            b[32] = order_float(hi);
           }
         }
       }
@@ -273,8 +274,10 @@ __global__ void __launch_bounds__(REFINE_THREADS) tree_refine_kernel(const T* __
       const uint32_t lo = __reduce_min_sync(FULL, lob[l * 32 + lane]);
       const uint32_t hi = __reduce_max_sync(FULL, hib[l * 32 + lane]);
       if (lane == 0) {
-        box[(uint64_t)(2 * l) * nodes + off1 + blockIdx.x] = order_float(lo);
-        box[(uint64_t)(2 * l + 1) * nodes + off1 + blockIdx.x] = order_float(hi);
+        const uint32_t node = off1 + blockIdx.x;
+        float* b = box + ((uint64_t)(node >> 5) * 2 * bd + 2 * l) * 32 + (node & 31u);
+        b[0] = order_float(lo);
+        b[32] = order_float(hi);
       }
     }
 }
@@ -284,21 +287,20 @@ struct TreeLevels {
   int levels;
   uint32_t count[TREE_MAX_LEVELS], offset[TREE_MAX_LEVELS];
 };
-__global__ void __launch_bounds__(1024) tree_upper_kernel(float* __restrict__ box, uint32_t nodes, uint32_t bd,
-                                                          const TreeLevels lv) {
+__global__ void __launch_bounds__(1024) tree_upper_kernel(float* __restrict__ box, uint32_t bd, const TreeLevels lv) {
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int h = 2; h < lv.levels; h++) {
     for (uint32_t w = warp; w < lv.count[h] * bd; w += 32) {
       const uint32_t l = w / lv.count[h], nd = w % lv.count[h];
-      const uint32_t ch = nd * 32 + lane;
-      const bool there = ch < lv.count[h - 1];
-      float* lo = box + (uint64_t)(2 * l) * nodes;
-      float* hi = lo + nodes;
-      const uint32_t a = __reduce_min_sync(FULL, there ? float_order(lo[lv.offset[h - 1] + ch]) : 0xffffffffu);
-      const uint32_t b = __reduce_max_sync(FULL, there ? float_order(hi[lv.offset[h - 1] + ch]) : 0u);
+      const bool there = nd * 32 + lane < lv.count[h - 1];
+      const float* in = box + ((uint64_t)((lv.offset[h - 1] >> 5) + nd) * 2 * bd + 2 * l) * 32 + lane;
+      const uint32_t a = __reduce_min_sync(FULL, there ? float_order(in[0]) : 0xffffffffu);
+      const uint32_t b = __reduce_max_sync(FULL, there ? float_order(in[32]) : 0u);
       if (lane == 0) {
-        lo[lv.offset[h] + nd] = order_float(a);
-        hi[lv.offset[h] + nd] = order_float(b);
+        const uint32_t node = lv.offset[h] + nd;
+        float* out = box + ((uint64_t)(node >> 5) * 2 * bd + 2 * l) * 32 + (node & 31u);
+        out[0] = order_float(a);
+        out[32] = order_float(b);
       }
     }
     __syncthreads();
@@ -343,7 +345,7 @@ void launch_tree_build(const T* xs, const T* minmax, uint64_t n, uint32_t d, Tre
   KNNSJ_CUDA(cudaFuncSetAttribute(tree_refine_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   tree_refine_kernel<T><<<(unsigned)((n + BLOCK_PTS - 1) / BLOCK_PTS), REFINE_THREADS, smem, s>>>(
       xs, n, d, rd, sc.sort.vals[cur], const_cast<T*>(t.ps), const_cast<float*>(t.psf), const_cast<uint32_t*>(t.id),
-      t.ld, const_cast<float*>(t.box), t.nodes, t.dims, t.count[0], t.levels > 1 ? t.offset[1] : 0xffffffffu);
+      const_cast<float*>(t.box), t.dims, t.count[0], t.levels > 1 ? t.offset[1] : 0xffffffffu);
   KNNSJ_CHECK_LAUNCH();
   if (t.levels > 2) {
     TreeLevels lv;
@@ -352,7 +354,7 @@ void launch_tree_build(const T* xs, const T* minmax, uint64_t n, uint32_t d, Tre
       lv.count[h] = t.count[h];
       lv.offset[h] = t.offset[h];
     }
-    tree_upper_kernel<<<1, 1024, 0, s>>>(const_cast<float*>(t.box), t.nodes, t.dims, lv);
+    tree_upper_kernel<<<1, 1024, 0, s>>>(const_cast<float*>(t.box), t.dims, lv);
     KNNSJ_CHECK_LAUNCH();
   }
 }

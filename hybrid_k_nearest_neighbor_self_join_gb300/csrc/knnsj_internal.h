@@ -137,7 +137,16 @@ void launch_cell_ids(const T* soa, uint64_t n, const GridGeom<T>& g, unsigned lo
                      uint32_t* vals, cudaStream_t s);
 // Stable LSD radix sort of (key, value) by the low `bits` bits of key.
 // Returns the index (0/1) of the buffers holding the result.
-int radix_sort_pairs(GridScratch& sc, uint64_t n, int bits, cudaStream_t s);
+// limit (optional, device): the largest key.  Passes above its highest digit
+// are skipped on the device: the result is then in the buffers of the last
+// pass that ran (index radix_passes(*limit) & 1), not in the returned ones.
+int radix_sort_pairs(GridScratch& sc, uint64_t n, int bits, cudaStream_t s,
+                     const unsigned long long* limit = nullptr);
+__host__ __device__ inline int radix_passes(unsigned long long limit) {
+  int p = 0;
+  for (; limit; limit >>= 8) p++;
+  return p;
+}
 // Non-empty cell table from sorted keys; writes C to *d_C.
 void launch_compact_cells(const unsigned long long* skeys, uint64_t n, uint32_t* flags,
                           uint32_t* pos, uint32_t* scan_tmp, unsigned long long* ckeys,
@@ -282,11 +291,13 @@ constexpr int TREE_MAX_LEVELS = 6;   // 32^6 leaves
 constexpr uint32_t TREE_DIMS = 16;   // dimensions the boxes cover (the first ones: largest variance)
 template <typename T>
 struct BoxTree {
-  const T* ps = nullptr;         // columns in tree order, stride ld
+  // Everything a warp reads at a time lies together, 32 lanes wide: a leaf's
+  // points are d rows of 32 coordinates, a node's children 2 * dims rows of 32
+  // bounds (one address and immediate offsets instead of one per row).
+  const T* ps = nullptr;         // [leaf][d][32]; the last leaf is filled up with infinities
   const float* psf = nullptr;    // double data: the same rounded to float (the float screen)
-  const uint32_t* id = nullptr;  // original id of each tree position
-  const float* box = nullptr;    // [2 * dims][nodes]: lower and upper bound of each dimension
-  uint64_t ld = 0;
+  const uint32_t* id = nullptr;  // original id of each tree position (filled up with 0xffffffff)
+  const float* box = nullptr;    // [node / 32][2 * dims][32]: lower and upper bound of each dimension
   uint32_t dims = 0;             // min(d, TREE_DIMS)
   uint32_t nodes = 0;
   int levels = 0;                // level 0: the leaves; the last level has at most 32 nodes

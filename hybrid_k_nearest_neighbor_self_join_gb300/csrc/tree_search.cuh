@@ -136,17 +136,18 @@ __device__ __noinline__ void tree_settle(const TreeParams<T>& p, TreeState<T, Q>
         if (lane < (int)cnt) {
           const uint32_t j = queue[i * TREE_QUEUE + qn + lane];
           const T* qc = qsm + (D > 0 ? i * D : i * (int)p.d);
+          const T* x = p.t.ps + (uint64_t)(j >> 5) * 32 * (D > 0 ? (uint32_t)D : p.d) + (j & 31u);
           T acc = 0;
           if (D > 0) {
 #pragma unroll
             for (int l = 0; l < (D > 0 ? D : 1); l++) {
-              const T t = Num<T>::sub(p.t.ps[(uint64_t)l * p.t.ld + j], qc[l]);
+              const T t = Num<T>::sub(x[l * 32], qc[l]);
               acc = Num<T>::fma(t, t, acc);
             }
           } else {
 #pragma unroll 4
             for (uint32_t l = 0; l < p.d; l++) {
-              const T t = Num<T>::sub(p.t.ps[(uint64_t)l * p.t.ld + j], qc[l]);
+              const T t = Num<T>::sub(x[l * 32], qc[l]);
               acc = Num<T>::fma(t, t, acc);
             }
           }
@@ -188,7 +189,7 @@ struct TreeTile {
   uint32_t len[Q], trig[Q];
   float qnorm[Q];    // double data: at least |q|
   uint32_t qn[Q];    // double: queue length
-  unsigned long long scanned = 0;
+  uint32_t scanned = 0;  // leaves scanned, per query
 
   __device__ __forceinline__ TreeTile(const TreeParams<T>& p_, int lane_) : p(p_), lane(lane_) {}
 
@@ -229,32 +230,35 @@ struct TreeTile {
   // The points of leaf c of a node for the queries whose masks pm hold bit c.
   // True when the shared state has changed.
   __device__ __forceinline__ bool scan_leaf(uint32_t leaf, int c, const unsigned (&pm)[Q]) {
-    const uint32_t held = (uint32_t)min(32ull, (unsigned long long)(p.n - (uint64_t)leaf * 32));
-    const bool valid = lane < (int)held;
-    const uint32_t j = valid ? leaf * 32 + lane : (uint32_t)p.n - 1;
-    const float* src = sizeof(T) == 4 ? reinterpret_cast<const float*>(p.t.ps) : p.t.psf;
-    const uint32_t id = sizeof(T) == 4 ? p.t.id[j] : 0u;
+    // (the points that fill up the last leaf lie at infinity, with an id that
+    // no threshold key exceeds)
+    const float* src = (sizeof(T) == 4 ? reinterpret_cast<const float*>(p.t.ps) : p.t.psf) +
+                       (uint64_t)leaf * 32 * (D > 0 ? (uint32_t)D : p.d) + lane;
     bool due = false;
     auto take = [&](int i, float a) {
-      if constexpr (sizeof(T) == 4) {
-        const bool pass = valid && (a < tauf[i] || (a == tauf[i] && id < tid[i]));
-        const unsigned m = __ballot_sync(FULL, pass);
-        if (pass) buf[(size_t)i * p.B + len[i] + __popc(m & lanemask_lt())] = Kt::make(a, id);
-        len[i] += __popc(m);
-        due |= len[i] > trig[i];
-      } else {
-        const bool pass = valid && a <= tauf[i];
-        const unsigned m = __ballot_sync(FULL, pass);
-        if (pass) queue[i * TREE_QUEUE + qn[i] + __popc(m & lanemask_lt())] = j;
-        qn[i] += __popc(m);
-        due |= qn[i] >= 32;
+      bool pass = a <= tauf[i];
+      unsigned m = __ballot_sync(FULL, pass);
+      scanned++;
+      if (m) {
+        if constexpr (sizeof(T) == 4) {
+          const uint32_t id = p.t.id[leaf * 32 + lane];
+          // (equal to the threshold distance: the smaller id passes)
+          pass = pass && (a < tauf[i] || id < tid[i]);
+          m = __ballot_sync(FULL, pass);
+          if (pass) buf[(size_t)i * p.B + len[i] + __popc(m & lanemask_lt())] = Kt::make(a, id);
+          len[i] += __popc(m);
+          due |= len[i] > trig[i];
+        } else {
+          if (pass) queue[i * TREE_QUEUE + qn[i] + __popc(m & lanemask_lt())] = leaf * 32 + lane;
+          qn[i] += __popc(m);
+          due |= qn[i] >= 32;
+        }
       }
-      scanned += held;
     };
     if (D > 0) {
       float x[QD];
 #pragma unroll
-      for (int l = 0; l < QD; l++) x[l] = src[(uint64_t)l * p.t.ld + j];
+      for (int l = 0; l < QD; l++) x[l] = src[l * 32];
 #pragma unroll
       for (int i = 0; i < Q; i++) {
         if (pm[i] >> c & 1u) {
@@ -273,7 +277,7 @@ struct TreeTile {
       for (int i = 0; i < Q; i++) acc[i] = 0.0f;
 #pragma unroll 4
       for (uint32_t l = 0; l < p.d; l++) {
-        const float x = src[(uint64_t)l * p.t.ld + j];
+        const float x = src[l * 32];
 #pragma unroll
         for (int i = 0; i < Q; i++) {
           const float t = __fsub_rn(x, qfm[l * Q + i]);
@@ -289,15 +293,16 @@ struct TreeTile {
   }
 
   // Lower bounds of the (float) squared distance from each query to the points
-  // in the box of this lane's child of a level (NaN: no such child).
-  __device__ __forceinline__ void box_bounds(uint32_t level, uint32_t child, float (&lb)[Q]) {
-    const bool there = child < p.t.count[level];
-    const uint32_t c = p.t.offset[level] + (there ? child : 0u);
+  // in the box of child lane ^ flip of a node, at `level` (NaN: no such child).
+  __device__ __forceinline__ void box_bounds(uint32_t level, uint32_t node, uint32_t flip, float (&lb)[Q]) {
+    const uint32_t c = lane ^ flip;
+    const bool there = node * 32 + c < p.t.count[level];
+    const float* box = p.t.box + (uint64_t)((p.t.offset[level] >> 5) + node) * 64 * (D > 0 ? (uint32_t)D : p.t.dims) + c;
 #pragma unroll
     for (int i = 0; i < Q; i++) lb[i] = 0.0f;
     auto dim = [&](uint32_t l, auto qof) {
-      const float lo = p.t.box[(uint64_t)(2 * l) * p.t.nodes + c];
-      const float hi = p.t.box[(uint64_t)(2 * l + 1) * p.t.nodes + c];
+      const float lo = box[l * 64];
+      const float hi = box[l * 64 + 32];
 #pragma unroll
       for (int i = 0; i < Q; i++) {
         const float v = qof(i);
@@ -330,7 +335,7 @@ struct TreeTile {
       // the order of the splits that part them from the own leaf)
       const uint32_t flip = level == 1 && top == 1 ? own & 31u : 0u;
       float lb[Q];
-      box_bounds(level - 1, node * 32 + (lane ^ flip), lb);
+      box_bounds(level - 1, node, flip, lb);
       float cur = none;  // level > 1: smallest bound over the queries that can use this lane's child
       if (level == 1) {
         unsigned pm[Q], todo = FULL;
@@ -456,14 +461,15 @@ __global__ void __launch_bounds__(TREE_THREADS, TREE_MIN_BLOCKS) tree_kernel(con
 #pragma unroll
     for (int i = 0; i < Q; i++) {
       const uint32_t at_pos = __shfl_sync(FULL, my_pos, i);
+      const uint64_t at0 = (uint64_t)own * 32 * (D > 0 ? (uint32_t)D : p.d) + (at_pos & 31u);
       if (D > 0) {
 #pragma unroll
         for (int l = 0; l < (D > 0 ? D : 1); l++)
-          t.q[i][l] = sizeof(T) == 8 ? p.t.psf[(uint64_t)l * p.t.ld + at_pos] : (float)p.t.ps[(uint64_t)l * p.t.ld + at_pos];
+          t.q[i][l] = sizeof(T) == 8 ? p.t.psf[at0 + l * 32] : (float)p.t.ps[at0 + l * 32];
       }
       if (sizeof(T) == 8 || D == 0) {
         for (uint32_t l = lane; l < p.d; l += 32) {
-          const T v = p.t.ps[(uint64_t)l * p.t.ld + at_pos];
+          const T v = p.t.ps[at0 + l * 32];
           if (sizeof(T) == 8) t.qsm[i * p.d + l] = v;
           if (D == 0) t.qfm[l * Q + i] = (float)v;
         }
@@ -524,7 +530,7 @@ __global__ void __launch_bounds__(TREE_THREADS, TREE_MIN_BLOCKS) tree_kernel(con
     }
   }
   if (lane == 0) {
-    if (t.scanned) atomicAdd(p.cand_count, t.scanned);
+    if (t.scanned) atomicAdd(p.cand_count, 32ull * t.scanned);
     if (rmax > (T)0)
       atomicMax(p.rmax_bits, (unsigned long long)Num<T>::bits(p.unbounded ? Num<T>::sqrt(rmax) : rmax));
   }
