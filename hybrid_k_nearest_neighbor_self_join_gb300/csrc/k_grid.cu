@@ -22,7 +22,11 @@ namespace {
 
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ITEMS = 16;                      // rounds of 32 keys per warp
+// (outlier scores of 2M rows / the 25M sky join with 16 rounds and 3 blocks
+// per SM 0.556 / 41.8 ms, 8 and 3 0.498 / 41.3, 8 and 4 0.487 / 41.1, 8 and 6
+// 0.520 / 41.4: latency of the ranking rounds, not the length of the runs)
+constexpr int RS_ITEMS = 8;                       // rounds of 32 keys per warp
+constexpr int RS_MIN_BLOCKS = 4;
 constexpr int RS_TILE = RS_THREADS * RS_ITEMS;    // keys per block tile
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
@@ -43,7 +47,7 @@ __global__ void cell_id_kernel(const T* __restrict__ soa, uint64_t n, const Grid
   }
 }
 
-// A radix pass is three launches: the digit counts of each tile of 4096 keys,
+// A radix pass is three launches: the digit counts of each tile of 2048 keys,
 // per digit the running sums over the tiles (one block per digit), and the
 // scatter, which sorts its tile by digit in shared memory first, so that a
 // digit's keys leave in one run.  (Scattering straight from registers wrote
@@ -125,11 +129,11 @@ __global__ void __launch_bounds__(RS_THREADS) radix_rows_kernel(uint32_t* __rest
   if (threadIdx.x == 0) total[blockIdx.x] = carry;
 }
 
-// Stable scatter: warp w owns keys [tile + 512 w, tile + 512 w + 512) and
+// Stable scatter: warp w owns keys [tile + 256 w, tile + 256 w + 256) and
 // visits them in order, 32 at a time; equal digits within a round are ranked
 // by lane, rounds by order, warps by index, tiles by the running sums.
 constexpr int RS_SMEM = RS_TILE * 12 + RS_WARPS * 256 * 4 + 256 * 4;
-__global__ void __launch_bounds__(RS_THREADS) radix_scatter_kernel(
+__global__ void __launch_bounds__(RS_THREADS, RS_MIN_BLOCKS) radix_scatter_kernel(
     const unsigned long long* __restrict__ kin, const uint32_t* __restrict__ vin,
     unsigned long long* __restrict__ kout, uint32_t* __restrict__ vout, uint64_t n, int shift, uint32_t ntiles,
     const uint32_t* __restrict__ rows, const uint32_t* __restrict__ total,
@@ -144,6 +148,7 @@ __global__ void __launch_bounds__(RS_THREADS) radix_scatter_kernel(
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < RS_WARPS * 256; i += RS_THREADS) wc[i] = 0;
   __syncthreads();
+  const uint32_t tot = total[threadIdx.x], row = rows[(uint64_t)threadIdx.x * ntiles + blockIdx.x];
   const uint64_t base = (uint64_t)blockIdx.x * RS_TILE;
   const uint64_t wbase = base + (uint64_t)w * (RS_ITEMS * 32);
   unsigned long long k[RS_ITEMS];
@@ -169,17 +174,19 @@ __global__ void __launch_bounds__(RS_THREADS) radix_scatter_kernel(
   __syncthreads();
   {
     const int digit = threadIdx.x;  // RS_THREADS == 256
-    uint32_t here = 0;
+    uint32_t c[RS_WARPS], here = 0, all;
+#pragma unroll
     for (int ww = 0; ww < RS_WARPS; ww++) {
-      const uint32_t c = wc[ww * 256 + digit];
-      wc[ww * 256 + digit] = here;
-      here += c;
+      c[ww] = wc[ww * 256 + digit];
+      here += c[ww];
     }
-    uint32_t all;
-    const uint32_t start = block_exclusive(here, ws, all);
-    const uint32_t global = block_exclusive(total[digit], ws, all) + rows[(uint64_t)digit * ntiles + blockIdx.x];
-    for (int ww = 0; ww < RS_WARPS; ww++) wc[ww * 256 + digit] += start;
-    gb[digit] = global - start;
+    uint32_t run = block_exclusive(here, ws, all);
+    gb[digit] = block_exclusive(tot, ws, all) + row - run;
+#pragma unroll
+    for (int ww = 0; ww < RS_WARPS; ww++) {
+      wc[ww * 256 + digit] = run;
+      run += c[ww];
+    }
   }
   __syncthreads();
 #pragma unroll

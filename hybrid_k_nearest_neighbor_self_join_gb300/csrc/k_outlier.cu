@@ -41,7 +41,8 @@ __global__ void in_degree_kernel(const int32_t* __restrict__ ids, uint64_t count
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const int32_t id = ids[i];
-    if (id >= 0 && (uint64_t)id < n) atomicAdd(&indeg[id], 1ull);
+    // (a degree is at most n < 2^31: its low word is counted)
+    if (id >= 0 && (uint64_t)id < n) atomicAdd(reinterpret_cast<uint32_t*>(&indeg[id]), 1u);
   }
 }
 
@@ -73,7 +74,8 @@ __global__ void degree_keys_kernel(const unsigned long long* __restrict__ indeg,
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, off));
-  if ((threadIdx.x & 31) == 0 && mx) atomicMax(largest, mx);
+  // (most warps see a larger value already there)
+  if ((threadIdx.x & 31) == 0 && mx > *(volatile unsigned long long*)largest) atomicMax(largest, mx);
 }
 
 // Ranks from the sort that stopped after the highest digit of *largest.
