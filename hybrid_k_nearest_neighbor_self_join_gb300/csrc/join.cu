@@ -125,6 +125,13 @@ void Workspace::release_all() {
   if (mail_host) cudaFreeHost(mail_host);
   mail_host = mail_dev = nullptr;
   mail = false;
+  if (stage) cudaFreeHost(stage);
+  stage = nullptr;
+  stage_blocks = 0;
+  for (auto& e : stage_ev) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  }
   pinned_release();
 }
 
@@ -163,6 +170,24 @@ void Workspace::ensure_mail() {
   if (mail_host || g_forbid_alloc) return;  // (fixed-scratch joins copy into pageable memory)
   KNNSJ_CUDA(cudaHostAlloc(&mail_host, MAIL_BYTES, cudaHostAllocMapped));
   KNNSJ_CUDA(cudaHostGetDevicePointer(&mail_dev, mail_host, 0));
+}
+
+bool Workspace::ensure_stage(int blocks) {
+  if (g_forbid_alloc) return false;
+  if (blocks > stage_blocks) {
+    if (stage) cudaFreeHost(stage);
+    stage = nullptr;
+    stage_blocks = 0;
+    if (cudaMallocHost(&stage, (size_t)blocks * STAGE_BYTES) != cudaSuccess) {
+      cudaGetLastError();
+      stage = nullptr;
+      return false;
+    }
+    stage_blocks = blocks;
+  }
+  for (int i = 0; i < blocks; i++)
+    if (!stage_ev[i]) KNNSJ_CUDA(cudaEventCreateWithFlags(&stage_ev[i], cudaEventDisableTiming));
+  return true;
 }
 
 namespace {

@@ -273,6 +273,10 @@ void launch_brute(const SearchLaunch<T>& a, cudaStream_t s);
 // the host buffers by a kernel at the end, after every chunk copy.
 constexpr int MAX_ROW_CHUNKS = 32;
 constexpr size_t MAIL_BYTES = 16384;  // mailbox: reads in the first half, writes in the second
+// Staging blocks of result tables on their way into pageable host buffers, one
+// per copying thread (up to 16 MB pinned per workspace).
+constexpr int STAGE_BLOCKS = 8;
+constexpr size_t STAGE_BYTES = 2u << 20;
 struct RowStream {
   void* ids_host = nullptr;  // the host buffers
   void* d_host = nullptr;
@@ -369,11 +373,15 @@ struct Workspace {
   void* mail_dev = nullptr;
   bool mail = false;
   int sm_count = 0;
+  void* stage = nullptr;                 // staging blocks (pinned) and their copies' events
+  int stage_blocks = 0;
+  cudaEvent_t stage_ev[STAGE_BLOCKS] = {};
   void* h_pinned = nullptr;
   size_t h_pinned_bytes = 0;
   void ensure_stream();
   void ensure_copy_stream();
   void ensure_mail();
+  bool ensure_stage(int blocks);  // false: no pinned memory to be had
   void* pinned(size_t need);
   void pinned_release();
   void release_all();
