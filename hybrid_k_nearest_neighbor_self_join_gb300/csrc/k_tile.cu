@@ -26,18 +26,13 @@
 //      a query that finds more keys than the list holds (0.2 % of the sky
 //      join) is handed to search_kernel, one that finds fewer than K fails
 //      (the reference's acceptance rule, GPU.cu:3659-3669);
-//   4. a histogram of the list in 128 bins of squared distance (a monotone
-//      map of [0, r^2]; 8-bit counts, four to a word, scanned bytewise),
-//      the bin holding the K-th smallest key and the count below it; a
-//      boundary bin with more keys than the 16-entry overflow list is split
-//      32 ways (at most two refinements; beyond, only exact ties, the query
-//      goes to search_kernel);
-//   5. placement: the list index of every key below the boundary bin goes
-//      to its bin's running slot of the row (a counting sort by bin), keys
-//      of the boundary bin to the overflow list; the few bins holding two
-//      keys or more are sorted, and so is the overflow list;
-//   6. the warp writes each query's row with coalesced stores (distances
-//      as sqrt in the data type), the first K - c_lo overflow keys last.
+//   4. each accepted query's list is sorted by the whole warp as 32-bit words
+//      (25 bits of squared distance over its list index), 4 per lane, in
+//      registers; words of equal distance bits are put in order of their full
+//      keys by passes over neighbours (few queries have any; one that needs
+//      more than SORT_FIXES passes is handed to search_kernel);
+//   5. the warp writes the row with coalesced stores (distances as sqrt in the
+//      data type).
 // Squared distances use the reference's fma chain in dimension order
 // (kernel.cu:139-140) exactly as search_kernel does, so rows are identical.
 // Keys are (squared distance bits, id) in one u64: ties are ordered by id.
@@ -54,9 +49,7 @@ namespace {
 constexpr int TILE_WARPS = 4;                    // warps per block
 constexpr int TILE_THREADS = TILE_WARPS * 32;
 constexpr int TILE_CH = 64;                      // staged candidates per chunk
-constexpr int TILE_BINS0 = 128;                  // level-0 bins (8-bit counts, four to a word)
-constexpr int TILE_BINS = 32;                    // bins of a refinement level (32-bit counts)
-constexpr int TILE_OV = 16;                      // overflow keys per query
+constexpr int SORT_FIXES = 24;                   // passes over neighbours of equal distance bits
 constexpr uint32_t TILE_MAX_ROWS = 4096;         // larger union boxes go to search_kernel
 
 struct alignas(16) Cand {
@@ -66,32 +59,21 @@ struct alignas(16) Cand {
 
 // Capacity of a query's key list: more than twice k+1 (the learned radius
 // finds 1.4 (k+1) keys on average; the few queries that find more are
-// handed to search_kernel: 1.1 % of the sky join with 132 entries for
-// k+1 = 65, about 0.2 % with 148, the most that 8 blocks of 4 warps of 4
-// queries leave room for), the pitch in u64 words = 4 (mod 16) so that the
-// lists of a warp's queries spread over the banks.
-constexpr int tile_list_cap(int kmax) { return kmax >= 65 ? 148 : kmax >= 33 ? 84 : 52; }
+// handed to search_kernel), the most that 8 blocks of 4 warps of 4 queries
+// leave room for, the pitch in u64 words = 4 (mod 16) so that the lists of a
+// warp's queries spread over the banks.
+constexpr int tile_list_cap(int kmax) { return kmax >= 65 ? 164 : kmax >= 33 ? 84 : 52; }
 
 // shared memory of one warp (bytes): QPT queries with rows of up to KMAX
-// keys.  The staging chunk, the refinement histograms and the rows' u16
-// list indices share one region (used one after another); a query's sorted
-// row is assembled at the start of its own list.
+// keys.  The staging chunk and the row's list indices share one region (used
+// one after the other).
 template <int QPT, int KMAX>
 struct TileSmem {
   static constexpr int C = tile_list_cap(KMAX);                 // list capacity per query (u64 keys)
-  static constexpr int HP = TILE_BINS + 1;                      // histogram pitch (u32 words)
-  static constexpr int RP = KMAX + 1;                           // row index pitch (u16)
-  static constexpr int SHARED_BYTES =
-      (TILE_CH * 16 > QPT * HP * 4 ? (TILE_CH * 16 > QPT * RP * 2 ? TILE_CH * 16 : QPT * RP * 2)
-                                   : (QPT * HP * 4 > QPT * RP * 2 ? QPT * HP * 4 : QPT * RP * 2));
+  static constexpr int R = C <= 64 ? 2 : 4;                     // words per lane of a sorted list
   static constexpr int LIST = 0;                                // [QPT][C] u64
-  static constexpr int CAND = LIST + QPT * C * 8;               // staging chunk | refinement bins | row indices
-  static constexpr int AUX = CAND;
-  static constexpr int RIDX = CAND;
-  static constexpr int HIST = (CAND + SHARED_BYTES + 15) / 16 * 16;  // [QPT][HP] u32
-  static constexpr int OVC = HIST + QPT * HP * 4;               // [QPT] u32 overflow counts
-  static constexpr int OVI = OVC + QPT * 4;                     // [QPT][TILE_OV] u16 overflow indices
-  static constexpr int RUNS = (OVI + QPT * TILE_OV * 2 + 15) / 16 * 16;  // 2 x 32 u32
+  static constexpr int CAND = LIST + QPT * C * 8;               // staging chunk | list indices
+  static constexpr int RUNS = CAND + TILE_CH * 16;              // 2 x 32 u32
   static constexpr int BYTES = RUNS + 2 * 32 * 4;
 };
 
@@ -122,13 +104,33 @@ struct TileParams {
   FailRadii* fail_radii;
 };
 
-// round(a * s + c) clamped to [0, NB - 1], with the integer read from the
-// low mantissa bits of a + 1.5 * 2^23 (one FMA); monotone in a.  c must be
-// an integer (exact in float).
-template <int NB>
-__device__ __forceinline__ int tbin(float a, float s, float cm) {
-  const int v = __float_as_int(__fmaf_rn(a, s, cm)) - 0x4b400000;
-  return min(max(v, 0), NB - 1);
+// Ascending bitonic sort of 32 R words across a warp; word i is v[i % R] of
+// lane i / R, so that the strides below R stay within a lane.
+template <int R>
+__device__ __forceinline__ void warp_sort_words(uint32_t (&v)[R], int lane) {
+#pragma unroll
+  for (int k = 2; k <= 32 * R; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j >= R) {
+        const bool keep_min = ((lane * R & k) == 0) == ((lane & (j / R)) == 0);
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          const uint32_t o = __shfl_xor_sync(FULL, v[r], j / R);
+          v[r] = keep_min ? min(v[r], o) : max(v[r], o);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          if (r & j) continue;
+          const bool up = k < R ? (r & k) == 0 : (lane * R & k) == 0;
+          const uint32_t lo = min(v[r], v[r | j]), hi = max(v[r], v[r | j]);
+          v[r] = up ? lo : hi;
+          v[r | j] = up ? hi : lo;
+        }
+      }
+    }
+  }
 }
 
 // Warp-aggregated append of this lane's value to a global list.
@@ -145,8 +147,7 @@ __device__ __forceinline__ void warp_append(bool want, uint32_t v, uint32_t* lis
 // QPT queries per warp (4, 8 or 16), LPQ = 32 / QPT lanes per query: lane
 // (slot qs = lane % QPT, phase ph = lane / QPT) evaluates the staged
 // candidates ph, ph + LPQ, ... for query qs.  The query's lanes share its
-// list, histogram, row indices and overflow list in shared memory; the lane
-// of phase 0 does the query's serial steps.  With 4 queries per warp the
+// list in shared memory; the lane of phase 0 does the query's serial steps.  With 4 queries per warp the
 // kernel is held to 64 registers: 8 blocks of 4 warps fit an SM.
 template <int D, int KMAX, int QPT>
 __global__ void __launch_bounds__(TILE_THREADS, QPT == 4 ? 8 : 5) tile_kernel(const TileParams p) {
@@ -162,12 +163,6 @@ __global__ void __launch_bounds__(TILE_THREADS, QPT == 4 ? 8 : 5) tile_kernel(co
   Cand* cand = reinterpret_cast<Cand*>(ws + SM::CAND);
   unsigned long long* lists = reinterpret_cast<unsigned long long*>(ws + SM::LIST);  // [QPT][C]
   unsigned long long* mylist = lists + (size_t)qs * SM::C;  // this query's keys, later its row
-  uint32_t* hq = reinterpret_cast<uint32_t*>(ws + SM::HIST) + qs * SM::HP;  // this query's bins
-  uint32_t* aq = reinterpret_cast<uint32_t*>(ws + SM::AUX) + qs * SM::HP;
-  uint16_t* rowix = reinterpret_cast<uint16_t*>(ws + SM::RIDX);  // [QPT][RP] list indices by row slot
-  uint32_t* ovcs = reinterpret_cast<uint32_t*>(ws + SM::OVC);
-  uint32_t* ovc = ovcs + qs;
-  uint16_t* ovi = reinterpret_cast<uint16_t*>(ws + SM::OVI);  // [QPT][TILE_OV] list indices
   uint32_t* runS = reinterpret_cast<uint32_t*>(ws + SM::RUNS);
   uint32_t* runP = runS + 32;
   // this query's lanes, and those of them below this lane
@@ -247,8 +242,6 @@ __global__ void __launch_bounds__(TILE_THREADS, QPT == 4 ? 8 : 5) tile_kernel(co
     warp_append(defer && lead, qid, p.defer_list, p.defer_count, lane);
 
     const float thr = in ? within_threshold(r) : -1.0f;  // acc <= thr never holds off the tile
-    const float s0 = (thr > 0.0f && thr < 3.0e38f) ? __fdividef((float)TILE_BINS0, thr) : 0.0f;
-    const float MAG = 12582912.0f;  // 1.5 * 2^23
 
     // Visits every candidate of the union box; body(c, live) runs on every
     // lane, live when c is a candidate of this lane's phase.
@@ -340,113 +333,6 @@ __global__ void __launch_bounds__(TILE_THREADS, QPT == 4 ? 8 : 5) tile_kernel(co
       }
       return acc;
     };
-    // zeroes a query's 32 histogram words (its LPQ lanes share the work)
-    auto clear_bins = [&](uint32_t* h) {
-      for (int b = ph; b < TILE_BINS; b += LPQ) h[b] = 0u;
-    };
-
-    // The boundary search over one query's 128 level-0 bins, 8-bit counts
-    // packed four to a word (h[w] holds bins 4w .. 4w+3; every count and
-    // every prefix is at most the list capacity, below 256, so bytewise sums
-    // never carry): each of the query's LPQ lanes takes 32 / LPQ consecutive
-    // words, one multiply by 0x01010101 gives a word's inclusive prefix per
-    // byte, a scan over the query's lanes gives each lane its starting
-    // count, and the bins become their exclusive prefix.  Outputs as for
-    // walk_bins below; `multi` gets a bit for each of this lane's bins
-    // (32 / LPQ words from bin 128 / LPQ * ph on) holding two keys or more.
-    auto walk_bytes = [&](uint32_t* h, uint32_t& total, uint32_t& lo_cnt, uint32_t& mb, uint32_t& bstar,
-                          unsigned long long& multi) {
-      constexpr int WPL = 32 / LPQ;
-      uint32_t wv[WPL];
-      uint32_t part = 0;
-      multi = 0;
-#pragma unroll
-      for (int i = 0; i < WPL; i++) {
-        wv[i] = h[ph * WPL + i];
-        part += (wv[i] * 0x01010101u) >> 24;
-        // bytes of 2 or more, 4 bits per word (a byte's carry only reaches
-        // bins above one of 130 keys or more, which lies at or above the
-        // boundary bin: the bins that get sorted hold fewer than K keys)
-        const uint32_t two = (wv[i] + 0x7e7e7e7eu) & 0x80808080u;
-        const uint32_t nib = ((two >> 7) & 1u) | ((two >> 14) & 2u) | ((two >> 21) & 4u) | ((two >> 28) & 8u);
-        multi |= (unsigned long long)nib << (4 * i);
-      }
-      uint32_t incl = part;
-#pragma unroll
-      for (int off = 1; off < LPQ; off <<= 1) {
-        const uint32_t tt = __shfl_up_sync(FULL, incl, off * QPT);
-        if (ph >= off) incl += tt;
-      }
-      uint32_t cum = incl - part;
-      uint32_t fb = TILE_BINS0, flo = 0, fm = 0;
-#pragma unroll
-      for (int i = 0; i < WPL; i++) {
-        const uint32_t w = wv[i];
-        const uint32_t pin = w * 0x01010101u;  // inclusive prefix within the word, per byte
-        h[ph * WPL + i] = (pin - w) + cum * 0x01010101u;
-        if (fb == TILE_BINS0 && cum + (pin >> 24) >= K) {
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const uint32_t cj = (pin >> (8 * j)) & 0xffu;
-            if (fb == TILE_BINS0 && cum + cj >= K) {
-              fb = (uint32_t)(4 * (ph * WPL + i) + j);
-              fm = (w >> (8 * j)) & 0xffu;
-              flo = cum + cj - fm;
-            }
-          }
-        }
-        cum += pin >> 24;
-      }
-      total = __shfl_sync(FULL, incl, qs + QPT * (LPQ - 1));
-      const unsigned hit = __ballot_sync(FULL, fb != TILE_BINS0);
-      const unsigned mine = hit & qmask;
-      const int src = mine ? __ffs(mine) - 1 : qs;
-      bstar = __shfl_sync(FULL, fb, src);
-      lo_cnt = __shfl_sync(FULL, flo, src);
-      mb = __shfl_sync(FULL, fm, src);
-    };
-
-    // The boundary search over one query's 32 bins (counts h[b], base keys
-    // below bin 0), shared by its LPQ lanes: each lane sums its 32 / LPQ
-    // consecutive bins, a scan over the query's lanes gives each lane its
-    // starting count, and the lane holding the bin where the count reaches K
-    // reports it.  With `prefix` the bins are replaced by their exclusive
-    // prefix (plus base).  Outputs are the query's (same on its lanes).
-    auto walk_bins = [&](uint32_t* h, uint32_t base, bool prefix, uint32_t& total, uint32_t& lo_cnt,
-                         uint32_t& mb, uint32_t& bstar) {
-      constexpr int BPL = TILE_BINS / LPQ;
-      uint32_t part = 0;
-#pragma unroll
-      for (int i = 0; i < BPL; i++) part += h[ph * BPL + i];
-      uint32_t incl = part;
-#pragma unroll
-      for (int off = 1; off < LPQ; off <<= 1) {
-        const uint32_t tt = __shfl_up_sync(FULL, incl, off * QPT);
-        if (ph >= off) incl += tt;
-      }
-      uint32_t cum = base + incl - part;
-      uint32_t fb = TILE_BINS, flo = 0, fm = 0;
-#pragma unroll
-      for (int i = 0; i < BPL; i++) {
-        const int b = ph * BPL + i;
-        const uint32_t hh = h[b];
-        if (prefix) h[b] = cum;
-        if (fb == TILE_BINS && cum + hh >= K) {
-          fb = (uint32_t)b;
-          flo = cum;
-          fm = hh;
-        }
-        cum += hh;
-      }
-      total = __shfl_sync(FULL, base + incl, qs + QPT * (LPQ - 1)) - base;
-      // the first lane of the query (by phase) that found the boundary
-      const unsigned hit = __ballot_sync(FULL, fb != TILE_BINS);
-      const unsigned mine = hit & qmask;
-      const int src = mine ? __ffs(mine) - 1 : qs;
-      bstar = __shfl_sync(FULL, fb, src);
-      lo_cnt = __shfl_sync(FULL, flo, src);
-      mb = __shfl_sync(FULL, fm, src);
-    };
 
     // 3. pass 1: every key within the radius is appended to the query's
     // list (slots from a ballot over the query's lanes: no atomics); the
@@ -466,178 +352,125 @@ __global__ void __launch_bounds__(TILE_THREADS, QPT == 4 ? 8 : 5) tile_kernel(co
     // a query with more keys than its list holds goes to search_kernel
     const bool big = in && found > (uint32_t)SM::C;
     warp_append(big && lead, qid, p.defer_list, p.defer_count, lane);
-    bool ok = in && found >= K && !big;
-    const uint32_t nl = ok ? found : 0u;  // list entries of an accepted query
+    const bool ok = in && found >= K && !big;
     __syncwarp();
 
-    // 128 bins of squared distance over the list (8-bit counts), the
-    // boundary bin of level 0 and the counts below it; the bins become their
-    // exclusive prefix
-    clear_bins(hq);
-    __syncwarp();
-    for (uint32_t e = (uint32_t)ph; e < nl; e += LPQ) {
-      const int b = tbin<TILE_BINS0>(__uint_as_float((uint32_t)(mylist[e] >> 32)), s0, MAG);
-      atomicAdd(&hq[b >> 2], 1u << (8 * (b & 3)));
-    }
-    __syncwarp();
-    uint32_t listed = 0, c_lo = 0, m = 0, bs0 = TILE_BINS0;
-    unsigned long long multi = 0;
-    walk_bytes(hq, listed, c_lo, m, bs0, multi);
-
-    // refinement of the boundary bin while it overflows the overflow list
-    int lev = 0;
-    int bs[3] = {(int)bs0, TILE_BINS, TILE_BINS};
-    float sl[3] = {s0, 0.0f, 0.0f}, cl[3] = {0.0f, 0.0f, 0.0f};  // scale and integer offset per level
+    // 4., 5. the accepted queries one after the other, by the whole warp
+    unsigned accepted = __ballot_sync(FULL, ok && lead);
+    while (accepted) {
+      const int rl = __ffs(accepted) - 1;  // (a lead lane: its index is the query slot)
+      accepted &= accepted - 1;
+      const uint32_t rid = __shfl_sync(FULL, qid, rl);
+      const uint32_t nl = __shfl_sync(FULL, found, rl);
+      const float top = __shfl_sync(FULL, thr, rl);
+      const unsigned long long* list = lists + (size_t)rl * SM::C;
+      uint32_t* words = reinterpret_cast<uint32_t*>(ws + SM::CAND);
+      constexpr int R = SM::R;
+      constexpr uint32_t NE = 32 * R, NONE = 0xffffffffu;
+      // word of a list entry: floor(acc * 2^25 / top), monotone in acc, over
+      // the entry's index
+      const float s25 = top > 0.0f && top < 3.0e38f ? __fdividef(33554400.0f, top) : 0.0f;
+      auto dist_bits = [&](uint32_t e) -> uint32_t {
+        const float acc = __uint_as_float((uint32_t)(list[e] >> 32));
+        return min(__float2uint_rz(acc * s25), 33554430u);
+      };
+      uint32_t v[R];
+      if (SM::C <= NE || nl <= NE) {
 #pragma unroll
-    for (int L = 1; L < 3; L++) {
-      const bool need = ok && lev == L - 1 && m > (uint32_t)TILE_OV;
-      if (!__any_sync(FULL, need)) break;
-      if (need) {
-        sl[L] = sl[L - 1] * (float)TILE_BINS;
-        cl[L] = (float)TILE_BINS * (cl[L - 1] - ((float)bs[L - 1] - 0.5f));
-        clear_bins(aq);
-      }
-      __syncwarp();
-      if (need) {
-        for (uint32_t e = (uint32_t)ph; e < nl; e += LPQ) {
-          const float acc = __uint_as_float((uint32_t)(mylist[e] >> 32));
-          if (tbin<TILE_BINS0>(acc, sl[0], MAG) != bs[0]) continue;
-          bool member = true;
+        for (int r = 0; r < R; r++) {
+          const uint32_t e = r * 32 + lane;
+          v[r] = e < nl ? dist_bits(e) << 7 | e : NONE;
+        }
+      } else {
+        // more keys than words (1 % of the sky join): those up to a distance
+        // that should leave between K and NE of them, their list indices
+        // closed up in shared memory
+        const uint32_t cut = (uint32_t)(33554432.0f * (0.5f * (float)(K + NE)) / (float)nl);
+        uint32_t kept = 0;
+        uint8_t* ix = reinterpret_cast<uint8_t*>(words) + NE;
+        for (uint32_t e0 = 0; e0 < nl; e0 += 32) {
+          const uint32_t e = e0 + lane;
+          const bool keep = e < nl && dist_bits(e) < cut;
+          const unsigned m = __ballot_sync(FULL, keep);
+          const uint32_t at = kept + __popc(m & lanemask_lt());
+          if (keep && at < NE) ix[at] = (uint8_t)e;
+          kept += __popc(m);
+        }
+        __syncwarp();
+        if (kept < K || kept > NE) {
+          if (lane == 0) p.defer_list[atomicAdd(p.defer_count, 1u)] = rid;
+          continue;
+        }
+        // (the words carry positions of the closed-up list)
 #pragma unroll
-          for (int l2 = 1; l2 < L; l2++)
-            if (tbin<TILE_BINS>(acc, sl[l2], MAG + cl[l2]) != bs[l2]) member = false;
-          if (member) atomicAdd(&aq[tbin<TILE_BINS>(acc, sl[L], MAG + cl[L])], 1u);
+        for (int r = 0; r < R; r++) {
+          const uint32_t e = r * 32 + lane;
+          v[r] = e < kept ? dist_bits(ix[e]) << 7 | e : NONE;
         }
       }
-      __syncwarp();
-      uint32_t nb = TILE_BINS, nlo = c_lo, nm = m, ntot = 0;
-      walk_bins(aq, c_lo, false, ntot, nlo, nm, nb);
-      if (need) {
-        bs[L] = (int)nb;
-        c_lo = nlo;
-        m = nm;
-        lev = L;
+      const bool closed = SM::C > NE && nl > NE;
+      const uint8_t* ix = reinterpret_cast<const uint8_t*>(words) + NE;
+      auto key_of = [&](uint32_t w) -> unsigned long long { return list[closed ? ix[w & 127u] : w & 127u]; };
+      warp_sort_words<R>(v, lane);
+      // neighbours of equal distance bits, in the order of their full keys
+      auto tied = [&](uint32_t a, uint32_t b) { return (a >> 7) == (b >> 7) && b != NONE; };
+      bool any = false;
+#pragma unroll
+      for (int r = 0; r + 1 < R; r++) any |= tied(v[r], v[r + 1]);
+      {
+        const uint32_t nx = __shfl_down_sync(FULL, v[0], 1);
+        any |= lane < 31 && tied(v[R - 1], nx);
       }
-      __syncwarp();
-    }
-    // still more boundary keys than the overflow list holds (exact ties):
-    // search_kernel takes the query
-    const bool tie_defer = ok && m > (uint32_t)TILE_OV;
-    warp_append(tie_defer && lead, qid, p.defer_list, p.defer_count, lane);
-    ok = ok && !tie_defer;
-
-    // 4. placement: the list index of every key below the boundary bin goes
-    // to its bin's running slot of the row (a counting sort by bin), the
-    // keys of the boundary bin to the overflow list
-    if (lead) *ovc = 0u;
-    __syncwarp();
-    if (ok) {
-      uint16_t* myridx = rowix + qs * SM::RP;
-      uint16_t* myovi = ovi + qs * TILE_OV;
-      for (uint32_t e = (uint32_t)ph; e < nl; e += LPQ) {
-        const float acc = __uint_as_float((uint32_t)(mylist[e] >> 32));
-        const int b0 = tbin<TILE_BINS0>(acc, sl[0], MAG);
-        bool place = b0 < bs[0];
-        bool over = b0 == bs[0] && lev == 0;
-        if (b0 == bs[0] && lev > 0) {  // (refined boundary bins only)
-          const int b1 = tbin<TILE_BINS>(acc, sl[1], MAG + cl[1]);
-          if (b1 < bs[1]) {
-            place = true;
-          } else if (b1 == bs[1]) {
-            if (lev == 1) {
-              over = true;
-            } else {
-              const int b2 = tbin<TILE_BINS>(acc, sl[2], MAG + cl[2]);
-              place = b2 < bs[2];
-              over = b2 == bs[2];
+      if (__any_sync(FULL, any)) {
+        int left = SORT_FIXES;
+        for (; left > 0; left--) {
+          bool moved = false;
+          auto order = [&](uint32_t& a, uint32_t& b) {
+            if (tied(a, b) && key_of(b) < key_of(a)) {
+              const uint32_t t2 = a;
+              a = b;
+              b = t2;
+              moved = true;
             }
-          }
+          };
+#pragma unroll
+          for (int r = 0; r + 1 < R; r += 2) order(v[r], v[r + 1]);
+#pragma unroll
+          for (int r = 1; r + 1 < R; r += 2) order(v[r], v[r + 1]);
+          // (both lanes of a pair take the same decision)
+          const uint32_t nx = __shfl_down_sync(FULL, v[0], 1), pv = __shfl_up_sync(FULL, v[R - 1], 1);
+          const bool give = lane < 31 && tied(v[R - 1], nx) && key_of(nx) < key_of(v[R - 1]);
+          const bool take = lane > 0 && tied(pv, v[0]) && key_of(v[0]) < key_of(pv);
+          if (give) v[R - 1] = nx;
+          if (take) v[0] = pv;
+          if (!__any_sync(FULL, moved || give || take)) break;
         }
-        if (place) {
-          const int sh = 8 * (b0 & 3);
-          myridx[(atomicAdd(&hq[b0 >> 2], 1u << sh) >> sh) & 0xffu] = (uint16_t)e;
+        if (left == 0) {  // too many equal distances
+          if (lane == 0) p.defer_list[atomicAdd(p.defer_count, 1u)] = rid;
+          continue;
         }
-        if (over) myovi[atomicAdd(ovc, 1u)] = (uint16_t)e;
       }
-    }
-    __syncwarp();
-
-    // 5. rows in order: after placement the byte of bin b <= bs0 holds the
-    // end of its slots (its start is the end of bin b - 1); only the bins
-    // the histogram found with two keys or more need ordering (the bins are
-    // narrow: 0.7 keys on average), and one lane sorts the overflow indices,
-    // whose smallest complete the row
-    auto isort_idx = [&](uint16_t* a, uint32_t lo, uint32_t hi) {
-      for (uint32_t i = lo + 1; i < hi; i++) {
-        const uint16_t ix = a[i];
-        const unsigned long long key = mylist[ix];
-        uint32_t j = i;
-        while (j > lo) {
-          const uint16_t pix = a[j - 1];
-          if (mylist[pix] <= key) break;
-          a[j] = pix;
-          j--;
-        }
-        a[j] = ix;
+      // list indices by row slot, four bytes to a word
+      uint32_t pack = 0;
+#pragma unroll
+      for (int r = 0; r < R; r++) pack |= (v[r] & 127u) << (8 * r);
+      uint8_t* slots = reinterpret_cast<uint8_t*>(words);
+      if (R == 4)
+        words[lane] = pack;
+      else
+        reinterpret_cast<uint16_t*>(words)[lane] = (uint16_t)pack;
+      __syncwarp();
+      const uint64_t base = (uint64_t)rid * K;
+      float rsq = 0.0f;
+      for (uint32_t s = (uint32_t)lane; s < K; s += 32) {
+        const unsigned long long key = key_of(slots[s]);
+        const float dist = __fsqrt_rn(__uint_as_float((uint32_t)(key >> 32)));
+        p.out_ids[base + s] = (int32_t)(uint32_t)key;
+        p.out_d[base + s] = dist;
+        rsq = __fadd_rn(rsq, __fmul_rn(dist, dist));
       }
-    };
-    auto sort_idx = [&](uint16_t* a, uint32_t lo, uint32_t hi) {
-      if (hi - lo == 2) {
-        const uint16_t i0 = a[lo], i1 = a[lo + 1];
-        if (mylist[i1] < mylist[i0]) {
-          a[lo] = i1;
-          a[lo + 1] = i0;
-        }
-      } else if (hi - lo > 2) {
-        isort_idx(a, lo, hi);
-      }
-    };
-    if (ok) {
-      constexpr int BPL = TILE_BINS0 / LPQ;  // bins per lane
-      uint16_t* myridx = rowix + qs * SM::RP;
-      // this lane's bins with placed keys: up to bs0 (bs0 itself only when
-      // refined: otherwise its keys are in the overflow list)
-      const int top = bs[0] - (lev == 0 ? 1 : 0) - BPL * ph;
-      unsigned long long mm = top < 0 ? 0ull : (top >= BPL - 1 ? multi : multi & ((2ull << top) - 1ull));
-      // a refined boundary bin is sorted whatever its count (a count above
-      // 129 would not show in the bytewise test)
-      if (lev > 0 && top >= 0 && top < BPL) mm |= 1ull << top;
-      while (mm) {
-        const int b = BPL * ph + __ffsll((long long)mm) - 1;
-        mm &= mm - 1;
-        const uint32_t w = hq[b >> 2];
-        const int j = b & 3;
-        const uint32_t hi = (w >> (8 * j)) & 0xffu;
-        const uint32_t lo = j ? (w >> (8 * (j - 1))) & 0xffu : (b ? hq[(b >> 2) - 1] >> 24 : 0u);
-        sort_idx(myridx, lo, hi);
-      }
-      if (ph == LPQ - 1) sort_idx(ovi + qs * TILE_OV, 0u, *ovc);
-    }
-    __syncwarp();
-    // coalesced row writes: the warp writes each accepted query's row, slot
-    // s from the list entry of row index s (s < c_lo) or of overflow index
-    // s - c_lo
-    {
-      unsigned mask = __ballot_sync(FULL, ok && lead);
-      while (mask) {
-        const int rl = __ffs(mask) - 1;  // (a lead lane: its index is the query slot)
-        mask &= mask - 1;
-        const uint32_t rid = __shfl_sync(FULL, qid, rl);
-        const uint32_t rclo = __shfl_sync(FULL, c_lo, rl);
-        const unsigned long long* rlist = lists + (size_t)rl * SM::C;
-        const uint16_t* rix = rowix + rl * SM::RP;
-        const uint16_t* rov = ovi + rl * TILE_OV;
-        const uint64_t base = (uint64_t)rid * K;
-        float rsq = 0.0f;
-        for (uint32_t s = (uint32_t)lane; s < K; s += 32) {
-          const unsigned long long key = rlist[s < rclo ? rix[s] : rov[s - rclo]];
-          const float dist = __fsqrt_rn(__uint_as_float((uint32_t)(key >> 32)));
-          p.out_ids[base + s] = (int32_t)(uint32_t)key;
-          p.out_d[base + s] = dist;
-          rsq = __fadd_rn(rsq, __fmul_rn(dist, dist));
-        }
-        if (p.rowsum) store_row_sum<float>(p.rowsum, rid, rsq, lane);
-      }
+      if (p.rowsum) store_row_sum<float>(p.rowsum, rid, rsq, lane);
+      __syncwarp();
     }
     // failures: fewer than K points within the radius
     const bool fail = in && found < K;
