@@ -76,66 +76,111 @@ __global__ void __launch_bounds__(SPLIT_THREADS) tree_split_kernel(const T* __re
 // dimensions, `bits` bits each (J. Skilling, "Programming the Hilbert curve",
 // 2004: Gray-code transpose, then the bits interleaved from the top).
 template <typename T>
+__device__ __forceinline__ unsigned long long curve_position(const T* __restrict__ xs, uint64_t n, uint64_t i,
+                                                             uint32_t hd, int bits, const float* sp) {
+  const float top = (float)(1u << bits);
+  uint32_t X[TREE_KEY_DIMS];
+#pragma unroll
+  for (uint32_t j = 0; j < TREE_KEY_DIMS; j++) {
+    X[j] = 0;
+    if (j < hd) {
+      const float v = (float)xs[(uint64_t)j * n + i];
+      const float* q = sp + j * (TREE_BINS + 1);
+      uint32_t lo = 0;  // last bin whose lower edge is <= v
+#pragma unroll
+      for (uint32_t step = TREE_BINS / 2; step > 0; step >>= 1)
+        if (q[lo + step] <= v) lo += step;
+      const float w = q[lo + 1] - q[lo];
+      float f = w > 0.0f ? (v - q[lo]) / w : 0.0f;
+      f = fminf(fmaxf(f, 0.0f), 0.999f);
+      X[j] = min((uint32_t)(((float)lo + f) * (top / (float)TREE_BINS)), (1u << bits) - 1u);
+    }
+  }
+  for (uint32_t m = 1u << (bits - 1); m > 1; m >>= 1) {
+    const uint32_t low = m - 1;
+#pragma unroll
+    for (uint32_t j = 0; j < TREE_KEY_DIMS; j++) {
+      if (j < hd) {
+        if (X[j] & m) {
+          X[0] ^= low;
+        } else {
+          const uint32_t t = (X[0] ^ X[j]) & low;
+          X[0] ^= t;
+          X[j] ^= t;
+        }
+      }
+    }
+  }
+  uint32_t last = 0;
+#pragma unroll
+  for (uint32_t j = 1; j < TREE_KEY_DIMS; j++)
+    if (j < hd) X[j] ^= X[j - 1];
+#pragma unroll
+  for (uint32_t j = 0; j < TREE_KEY_DIMS; j++)
+    if (j + 1 == hd) last = X[j];
+  uint32_t t = 0;
+  for (uint32_t m = 1u << (bits - 1); m > 1; m >>= 1)
+    if (last & m) t ^= m - 1;
+  unsigned long long code = 0;
+  for (int b = bits - 1; b >= 0; b--) {
+#pragma unroll
+    for (uint32_t j = 0; j < TREE_KEY_DIMS; j++)
+      if (j < hd) code = (code << 1) | (((X[j] ^ t) >> b) & 1u);
+  }
+  return code;
+}
+
+template <typename T>
 __global__ void tree_key_kernel(const T* __restrict__ xs, uint64_t n, uint32_t hd, int bits,
                                 const float* __restrict__ split, unsigned long long* __restrict__ keys,
                                 uint32_t* __restrict__ vals) {
   __shared__ float sp[TREE_KEY_DIMS * (TREE_BINS + 1)];
   for (uint32_t i = threadIdx.x; i < hd * (TREE_BINS + 1); i += blockDim.x) sp[i] = split[i];
   __syncthreads();
-  const float top = (float)(1u << bits);
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t X[TREE_KEY_DIMS];
-#pragma unroll
-    for (uint32_t j = 0; j < TREE_KEY_DIMS; j++) {
-      X[j] = 0;
-      if (j < hd) {
-        const float v = (float)xs[(uint64_t)j * n + i];
-        const float* q = sp + j * (TREE_BINS + 1);
-        uint32_t lo = 0;  // last bin whose lower edge is <= v
-#pragma unroll
-        for (uint32_t step = TREE_BINS / 2; step > 0; step >>= 1)
-          if (q[lo + step] <= v) lo += step;
-        const float w = q[lo + 1] - q[lo];
-        float f = w > 0.0f ? (v - q[lo]) / w : 0.0f;
-        f = fminf(fmaxf(f, 0.0f), 0.999f);
-        X[j] = min((uint32_t)(((float)lo + f) * (top / (float)TREE_BINS)), (1u << bits) - 1u);
-      }
-    }
-    for (uint32_t m = 1u << (bits - 1); m > 1; m >>= 1) {
-      const uint32_t low = m - 1;
-#pragma unroll
-      for (uint32_t j = 0; j < TREE_KEY_DIMS; j++) {
-        if (j < hd) {
-          if (X[j] & m) {
-            X[0] ^= low;
-          } else {
-            const uint32_t t = (X[0] ^ X[j]) & low;
-            X[0] ^= t;
-            X[j] ^= t;
-          }
-        }
-      }
-    }
-    uint32_t last = 0;
-#pragma unroll
-    for (uint32_t j = 1; j < TREE_KEY_DIMS; j++)
-      if (j < hd) X[j] ^= X[j - 1];
-#pragma unroll
-    for (uint32_t j = 0; j < TREE_KEY_DIMS; j++)
-      if (j + 1 == hd) last = X[j];
-    uint32_t t = 0;
-    for (uint32_t m = 1u << (bits - 1); m > 1; m >>= 1)
-      if (last & m) t ^= m - 1;
-    unsigned long long code = 0;
-    for (int b = bits - 1; b >= 0; b--) {
-#pragma unroll
-      for (uint32_t j = 0; j < TREE_KEY_DIMS; j++)
-        if (j < hd) code = (code << 1) | (((X[j] ^ t) >> b) & 1u);
-    }
-    keys[i] = code;
+    keys[i] = curve_position(xs, n, i, hd, bits, sp);
     vals[i] = (uint32_t)i;
   }
+}
+
+// Up to SMALL_PTS points: positions and their sort in one block (10 launches
+// of a radix sort otherwise, 30 us of a join of 2000 points).  The codes have
+// at most 27 bits here.
+constexpr int SMALL_PTS = 4096;
+template <typename T>
+__global__ void __launch_bounds__(SPLIT_THREADS) tree_small_order_kernel(const T* __restrict__ xs, uint32_t n,
+                                                                         uint32_t hd, int bits,
+                                                                         const float* __restrict__ split,
+                                                                         uint32_t* __restrict__ vals) {
+  __shared__ float sp[TREE_KEY_DIMS * (TREE_BINS + 1)];
+  __shared__ unsigned long long key[SMALL_PTS];
+  for (uint32_t i = threadIdx.x; i < hd * (TREE_BINS + 1); i += blockDim.x) sp[i] = split[i];
+  __syncthreads();
+  uint32_t n2 = 64;
+  while (n2 < n) n2 <<= 1;
+  for (uint32_t i = threadIdx.x; i < n2; i += SPLIT_THREADS)
+    key[i] = i < n ? curve_position(xs, n, i, hd, bits, sp) << 12 | i : ~0ull;
+  __syncthreads();
+  for (uint32_t size = 2; size <= n2; size <<= 1) {
+    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+      for (uint32_t i = threadIdx.x; i < (n2 >> 1); i += SPLIT_THREADS) {
+        const uint32_t lo = ((i & ~(stride - 1)) << 1) | (i & (stride - 1));
+        const unsigned long long a = key[lo], b = key[lo + stride];
+        if ((b < a) == ((lo & size) == 0)) {
+          key[lo] = b;
+          key[lo + stride] = a;
+        }
+      }
+      // (a warp's pairs span 64 consecutive keys once the stride is at most 32)
+      if (stride > 32)
+        __syncthreads();
+      else
+        __syncwarp();
+    }
+    __syncthreads();
+  }
+  for (uint32_t i = threadIdx.x; i < n; i += SPLIT_THREADS) vals[i] = (uint32_t)key[i] & (SMALL_PTS - 1);
 }
 
 // floats as unsigned integers of the same order
@@ -336,10 +381,16 @@ void launch_tree_build(const T* xs, const T* minmax, uint64_t n, uint32_t d, Tre
   while (log2n < 31 && (1ull << log2n) < n) log2n++;
   int bits = (log2n + 8 + (int)hd - 1) / (int)hd;
   bits = std::max(2, std::min({bits, 16, (int)(60 / hd)}));
-  const unsigned blocks = (unsigned)std::min<uint64_t>((n + 255) / 256, 152ull * 32);
-  tree_key_kernel<T><<<blocks, 256, 0, s>>>(xs, n, hd, bits, sc.split, sc.sort.keys[0], sc.sort.vals[0]);
-  KNNSJ_CHECK_LAUNCH();
-  const int cur = radix_sort_pairs(sc.sort, n, bits * (int)hd, s);
+  int cur = 0;
+  if (n <= SMALL_PTS) {
+    tree_small_order_kernel<T><<<1, SPLIT_THREADS, 0, s>>>(xs, (uint32_t)n, hd, bits, sc.split, sc.sort.vals[0]);
+    KNNSJ_CHECK_LAUNCH();
+  } else {
+    const unsigned blocks = (unsigned)std::min<uint64_t>((n + 255) / 256, 152ull * 32);
+    tree_key_kernel<T><<<blocks, 256, 0, s>>>(xs, n, hd, bits, sc.split, sc.sort.keys[0], sc.sort.vals[0]);
+    KNNSJ_CHECK_LAUNCH();
+    cur = radix_sort_pairs(sc.sort, n, bits * (int)hd, s);
+  }
   const uint32_t rd = std::min<uint32_t>(d, REFINE_DIMS);
   const size_t smem = (size_t)rd * BLOCK_PTS * 4;
   KNNSJ_CUDA(cudaFuncSetAttribute(tree_refine_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
