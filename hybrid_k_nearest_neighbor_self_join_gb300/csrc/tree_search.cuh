@@ -40,7 +40,10 @@ namespace knnsj {
 namespace {
 
 constexpr int TREE_THREADS = 256;  // largest block
-constexpr int TREE_MIN_BLOCKS = 3;  // per SM: 80 registers
+// blocks per SM: 80 registers, and 64 in three dimensions (1M points: 4.5 and
+// 4.2 ms; two dimensions 11.2 and 11.1 ms at 3M but 0.21 and 0.22 at 100 000;
+// six spill: 147 and 187 ms)
+constexpr int tree_min_blocks(int d) { return d == 3 ? 4 : 3; }
 constexpr int TREE_Q = 2;          // queries per warp (1 with selection buffers above HIST_MAX_B)
 constexpr int TREE_QUEUE = 64;     // double data: candidates that passed the float screen, per query
 constexpr int TREE_STACK = 6;      // levels above the leaves' parents
@@ -402,7 +405,7 @@ __device__ __forceinline__ uint32_t nth_bit(unsigned w, uint32_t k) {
 }
 
 template <typename T, int D, int Q>
-__global__ void __launch_bounds__(TREE_THREADS, TREE_MIN_BLOCKS) tree_kernel(const TreeParams<T> p) {
+__global__ void __launch_bounds__(TREE_THREADS, tree_min_blocks(D)) tree_kernel(const TreeParams<T> p) {
   using Kt = Key<T>;
   using KT = typename Kt::type;
   extern __shared__ __align__(16) unsigned char smem[];
