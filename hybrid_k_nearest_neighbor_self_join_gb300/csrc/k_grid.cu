@@ -14,6 +14,8 @@
 // When the grid is small enough a dense start table replaces the binary
 // search over non-empty cells.
 
+#include <algorithm>
+
 #include "knnsj_internal.h"
 
 namespace knnsj {
@@ -421,8 +423,12 @@ template <typename T>
 __device__ __forceinline__ unsigned long long cell_of(const T* __restrict__ src, uint64_t n, uint64_t i,
                                                       const GridGeom<T>& g) {
   unsigned long long lin = 0;
+  // (clamped: where the cell width is below the rounding of the coordinates a
+  // point at the far edge divides out to the number of cells; the rings clamp
+  // their ends the same way)
   for (uint32_t j = 0; j < g.di; j++)
-    lin += (unsigned long long)point_cell_coord(src[(uint64_t)j * n + i], g.minv[j], g.width) * g.mult[j];
+    lin += (unsigned long long)min(point_cell_coord(src[(uint64_t)j * n + i], g.minv[j], g.width), g.ncell[j] - 1u) *
+           g.mult[j];
   return lin;
 }
 
@@ -472,8 +478,7 @@ __global__ void cell_mark_kernel(const T* __restrict__ soa, uint64_t n, const Gr
                                  uint32_t* __restrict__ bitmap, unsigned long long* __restrict__ count) {
   uint32_t fresh = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    // (never past the bitmap, whatever the rounding at the grid's far edge)
-    const unsigned long long lin = min(cell_of(soa, n, i, g), g.total_cells - 1ull);
+    const unsigned long long lin = cell_of(soa, n, i, g);
     const uint32_t bit = 1u << (lin & 31u);
     uint32_t* w = &bitmap[lin >> 5];
     // (a stale 0 only costs an atomic)
@@ -482,6 +487,16 @@ __global__ void cell_mark_kernel(const T* __restrict__ soa, uint64_t n, const Gr
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) fresh += __shfl_xor_sync(FULL, fresh, off);
   if ((threadIdx.x & 31) == 0 && fresh) atomicAdd(count, (unsigned long long)fresh);
+}
+
+__global__ void table_count_kernel(const uint32_t* __restrict__ dstart, unsigned long long total,
+                                   unsigned long long* __restrict__ count) {
+  uint32_t c = 0;
+  for (unsigned long long L = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; L < total;
+       L += (unsigned long long)gridDim.x * blockDim.x)
+    c += dstart[L + 1] != dstart[L] ? 1u : 0u;
+  c = __reduce_add_sync(FULL, c);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, (unsigned long long)c);
 }
 
 unsigned grid_blocks(uint64_t n, int threads = 256) {
@@ -576,6 +591,11 @@ void launch_counting_grid(const T* src, const uint32_t* src_ids, uint64_t n, uin
   KNNSJ_CHECK_LAUNCH();
   scan_exclusive_u32(tbl + 1, tbl + 1, g.total_cells, scan_tmp, s);
   cell_scatter_atomic_kernel<T><<<grid_blocks(n), 256, 0, s>>>(src, src_ids, n, d, g, tbl, ps, pid);
+  KNNSJ_CHECK_LAUNCH();
+}
+
+void launch_count_table(const uint32_t* dstart, unsigned long long total, unsigned long long* d_C, cudaStream_t s) {
+  table_count_kernel<<<(unsigned)std::min<unsigned>(grid_blocks(total), 152u * 8), 256, 0, s>>>(dstart, total, d_C);
   KNNSJ_CHECK_LAUNCH();
 }
 

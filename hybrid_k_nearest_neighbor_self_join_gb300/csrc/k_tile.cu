@@ -86,8 +86,7 @@ struct TileParams {
   uint32_t K;
   const float* __restrict__ qps;        // query columns: cell order (qlist null) or input order
   const uint32_t* __restrict__ qpid;    // ids of qps positions (qlist null)
-  const uint32_t* __restrict__ qlist;   // query ids, or null: the positions of qps in qorder
-  const uint32_t* __restrict__ qorder;  // positions of qps in tile order (null: 0, 1, ...)
+  const uint32_t* __restrict__ qlist;   // query ids, or null: the positions of qps
   uint32_t nq;
   float radius;                         // uniform radius (qradius null)
   float* qradius;                       // per-query radius by id
@@ -195,9 +194,8 @@ __global__ void __launch_bounds__(TILE_THREADS, QPT == 4 ? 8 : 5) tile_kernel(co
 #pragma unroll
     for (int j = 0; j < D; j++) q[j] = 0.0f;
     if (valid) {
-      const uint32_t pos = p.qorder ? p.qorder[qi] : qi;
-      qid = p.qlist ? p.qlist[qi] : p.qpid[pos];
-      const uint64_t col = p.qlist ? (uint64_t)qid : (uint64_t)pos;
+      qid = p.qlist ? p.qlist[qi] : p.qpid[qi];
+      const uint64_t col = p.qlist ? (uint64_t)qid : (uint64_t)qi;
 #pragma unroll
       for (int j = 0; j < D; j++) q[j] = p.qps[(uint64_t)j * n + col];
       r = p.qradius ? p.qradius[qid] : p.radius;
@@ -534,7 +532,6 @@ void launch_tile_search(const SearchLaunch<T>& a, uint32_t* defer_list, uint32_t
     p.qlist = a.qlist;
     p.qps = a.qlist ? a.xs : (a.qps ? a.qps : a.grid.ps);
     p.qpid = a.qps ? a.qpid : a.grid.pid;
-    p.qorder = a.qlist ? nullptr : a.qorder;
     p.nq = a.nq;
     p.radius = a.radius;
     p.qradius = a.qradius;

@@ -170,6 +170,8 @@ void launch_morton_keys(const T* ps, uint64_t n, const GridGeom<T>& g, int bits,
 template <typename T>
 void launch_counting_grid(const T* src, const uint32_t* src_ids, uint64_t n, uint32_t d, const GridGeom<T>& g,
                           uint32_t* tbl, uint32_t* scan_tmp, T* ps, uint32_t* pid, cudaStream_t s);
+// Number of cells with a point in a dense start table of `total` cells into *d_C.
+void launch_count_table(const uint32_t* dstart, unsigned long long total, unsigned long long* d_C, cudaStream_t s);
 template <typename T>
 // psf (optional): the same columns rounded to float (double data: the
 // search's float prefilter)
@@ -241,11 +243,10 @@ struct SearchLaunch {
   SearchShape shape;                        // launch shape (autotuned for batched joins)
   const LoopCtl* ctl = nullptr;             // non-null: nq, lists and radius come from here (graph passes)
   const uint32_t* nq_dev = nullptr;         // non-null: the pass's query count is read here (nq is a bound)
-  // tile search only: queries from these cell-ordered columns and ids (when
-  // the candidates come from another grid), visited in qorder
+  // tile search only: queries from these columns and ids, in tile order (when
+  // the candidates come from another grid)
   const T* qps = nullptr;
   const uint32_t* qpid = nullptr;
-  const uint32_t* qorder = nullptr;
 };
 template <typename T>
 void launch_search(const SearchLaunch<T>& a, int sm_count, cudaStream_t s);
@@ -358,7 +359,7 @@ struct Workspace {
   DevBuf rowsum;                         // per-row verification sums (host-pointer calls)
   DevBuf fps, fpid, fdstart;             // tile search: the finer candidate grid (columns, ids, start table)
   DevBuf tree_box, tree_split;           // box tree: node boxes, quantiles (points and ids in ps, psf, pid)
-  DevBuf qorder;                         // tile search: cell-ordered positions in Morton order of their cells
+  DevBuf curve_ps;                       // tile search: columns along the space-filling curve
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[8] = {};
   cudaStream_t copy_stream = nullptr;    // streamed rows: device-to-host copies
