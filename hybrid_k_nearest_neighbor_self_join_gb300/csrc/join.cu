@@ -770,12 +770,17 @@ struct Prepared {
 //   two dimensions, learned radii: rings of a few cells, few failures.  The
 //     tile kernel (float, k + 1 <= 65) 0.5-0.9x at 3 M; one warp per query
 //     0.9-1.2x below a million points, 1.04-1.36x at 3 M.
+//   k + 1 above 224 (float) or 192 (double): the selection buffer of 256 keys
+//     is reduced too often, and larger ones are sorted whole; 100 000-300 000
+//     points, k = 200: 1.06-5.7x float, 0.88-4.6x double, k = 223 double
+//     0.7-2.1x, k = 1000 0.65-1.0x, k = 4000 0.5-0.7x.
 constexpr uint64_t TREE_LEARNED_2D_MIN = 1000000;
 template <typename T>
 static bool tree_applies(const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t di, uint32_t K, double max_abs,
                          bool will_stream) {
   if (!cfg.tree_search || will_stream || cfg.max_iterations > 0) return false;
   if (sizeof(T) == 8 && (!cfg.float_prefilter || !(4.0 * std::sqrt((double)d) * max_abs < 1e18))) return false;
+  if (K > tree_max_k(sizeof(T))) return false;
   if (cfg.tree_search == 2) return true;
   if (cfg.tile_search >= 2) return false;
   if (d >= 3 || cfg.radius_mode != KNNSJ_RADIUS_LEARNED) return true;

@@ -316,6 +316,8 @@ struct TreeScratch {
 constexpr uint32_t TREE_KEY_DIMS = 8;    // dimensions of the space-filling curve
 constexpr uint32_t TREE_BINS = 256;      // quantile bins per dimension
 constexpr size_t tree_split_elems() { return (size_t)TREE_KEY_DIMS * (TREE_BINS + 1); }
+// Largest k+1 of a tree search (its selection buffers hold 256 keys).
+constexpr uint32_t tree_max_k(size_t elem) { return elem == 4 ? 224 : 192; }
 inline uint64_t tree_stride(uint64_t n) { return (n + 31) & ~31ull; }
 void tree_shape(uint64_t n, uint32_t d, uint32_t* count, uint32_t* offset, int* levels, uint32_t* nodes);
 // Builds the tree of the n points given as input-order columns xs (stride n)

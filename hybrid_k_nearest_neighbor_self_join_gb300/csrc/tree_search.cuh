@@ -44,7 +44,7 @@ constexpr int TREE_THREADS = 256;  // largest block
 // 4.2 ms; two dimensions 11.2 and 11.1 ms at 3M but 0.21 and 0.22 at 100 000;
 // six spill: 147 and 187 ms)
 constexpr int tree_min_blocks(int d) { return d == 3 ? 4 : 3; }
-constexpr int TREE_Q = 2;          // queries per warp (1 with selection buffers above HIST_MAX_B)
+constexpr int TREE_Q = 2;          // queries per warp
 constexpr int TREE_QUEUE = 64;     // double data: candidates that passed the float screen, per query
 constexpr int TREE_STACK = 6;      // levels above the leaves' parents
 constexpr uint32_t TREE_CHUNK = 64;  // tiles of a block's run of consecutive queries
@@ -510,10 +510,7 @@ __global__ void __launch_bounds__(TREE_THREADS, tree_min_blocks(D)) tree_kernel(
       const uint32_t id = p.t.id[at_pos];
       if (len >= p.K) {
         const uint64_t row = (uint64_t)id * p.K;
-        if (p.B <= HIST_MAX_B)
-          write_sorted_row<T>(buf, t.hist, len, tau, p.K, p.out_ids, p.out_d, row, lane, p.rowsum);
-        else
-          write_sorted_row_bitonic<T>(buf, len, p.K, p.out_ids, p.out_d, row, lane, p.rowsum);
+        write_sorted_row<T>(buf, t.hist, len, tau, p.K, p.out_ids, p.out_d, row, lane, p.rowsum);
         if (p.unbounded) {
           const T a = Kt::acc(tau);
           rmax = a > rmax ? a : rmax;
@@ -587,11 +584,9 @@ void launch_tree_search(const TreeLaunch<T>& a, int sm_count, cudaStream_t s) {
   p.n = a.n;
   p.d = a.d;
   p.K = a.K;
-  // selection buffer: room for K keys, what comes in between two reductions
-  // and a full leaf
-  uint32_t b = a.K <= 48 ? 128u : 256u;
-  while (b < a.K + 32) b <<= 1;
-  p.B = b;
+  // selection buffer: room for K <= tree_max_k keys, what comes in between two
+  // reductions and a full leaf
+  p.B = a.K <= 48 ? 128u : HIST_MAX_B;
   p.qmask = a.qmask;
   p.nq_dev = a.nq_dev;
   p.radius = a.radius;
@@ -606,10 +601,7 @@ void launch_tree_search(const TreeLaunch<T>& a, int sm_count, cudaStream_t s) {
   p.grow = a.grow;
   p.rmax_bits = a.rmax_bits;
   p.cand_count = a.cand_count;
-  if (b <= HIST_MAX_B)
-    launch_tree_d<T, TREE_Q>(p, sm_count, s);
-  else
-    launch_tree_d<T, 1>(p, sm_count, s);
+  launch_tree_d<T, TREE_Q>(p, sm_count, s);
 }
 
 }  // namespace knnsj

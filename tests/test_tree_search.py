@@ -80,3 +80,29 @@ def test_far_outliers_and_clumps(monkeypatch, dtype):
     far = rng.uniform(-1.0, 1.0, (9, 3)) * 20.0
     x = np.concatenate([c, c[:4_000] * 1e-2 + 0.5, far]).astype(dtype)
     check(monkeypatch, x, 16, queries=np.arange(16_000, 16_009))
+
+
+@pytest.mark.parametrize("d,dtype,mode", [(8, np.float64, kj.RADIUS_LEARNED), (8, np.float64, kj.RADIUS_PLAIN),
+                                          (2, np.float64, kj.RADIUS_PLAIN), (3, np.float32, kj.RADIUS_LEARNED)])
+def test_fixed_scratch_at_its_limits(d, dtype, mode):
+    # the largest problem of the fixed scratch array: grid, tree and radii all
+    # come from it
+    torch = pytest.importorskip("torch")
+    import ctypes
+    from hybrid_k_nearest_neighbor_self_join_gb300 import _lib
+    n, k = 65_536, 127
+    x = datasets.gmm(n, d, 9, 0.3, 60 + d, dtype=dtype)
+    dev = torch.from_numpy(x).cuda()
+    ids = [torch.full((n, k + 1), -7, dtype=torch.int32, device="cuda") for _ in range(2)]
+    dists = [torch.full((n, k + 1), -1.0, dtype=dev.dtype, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    opts = _lib.Options.make(radius_mode=mode)
+    code = _lib.KNNSJ_F32 if dtype == np.float32 else _lib.KNNSJ_F64
+    args = [ctypes.c_void_p(dev.data_ptr()), code, n, d, k, ctypes.byref(opts)]
+    lib = _lib.load()
+    _lib.check(lib.knnsj_selfjoin_device_noalloc(*args, ctypes.c_void_p(ids[0].data_ptr()),
+                                                 ctypes.c_void_p(dists[0].data_ptr())))
+    st = _lib.Stats.make()
+    _lib.check(lib.knnsj_selfjoin_device(*args, ctypes.c_void_p(ids[1].data_ptr()),
+                                         ctypes.c_void_p(dists[1].data_ptr()), ctypes.byref(st)))
+    assert torch.equal(ids[0], ids[1]) and torch.equal(dists[0], dists[1])
