@@ -2,10 +2,11 @@
 // of a tile of queries by one warp.  Compiled once per data type
 // (k_tree_f32.cu, k_tree_f64.cu).
 //
-// A warp owns Q queries of one leaf.  From that leaf it goes up the tree: the 32 children of a node are tested 32
-// lanes at a time against every query of the tile, the boxes that can hold a
-// point under a query's threshold are descended, and a leaf's 32 points are
-// loaded once and evaluated for each query that needs them.  A query's
+// A warp owns Q queries of one leaf.  From that leaf it goes up the tree: the
+// 32 children of a node are tested 32 lanes at a time against every query of
+// the tile, the boxes that can hold a point under a query's threshold are
+// descended, and a leaf's 32 points are loaded once and evaluated for each
+// query that needs them.  A query's
 // threshold starts at its radius (or without bound) and falls as its buffer
 // of keys is reduced to the K best.
 //
@@ -19,15 +20,15 @@
 // what passes gets its distance in double, 32 points at a time.
 //
 // What bounds it: issue slots and latency at 24 warps per SM (80 registers),
-// not memory (L2 hits 97 %, DRAM idle): about 5 700 warp instructions per query
-// of a 6-D double join at 0.42 per cycle and scheduler, half of them on the
-// ~65 leaves a query visits.  Search kernels of whole joins, one warp per query
-// on the grid's ring (k_search.cu) before, this now: 10 M x 6-D double k = 16
-// 790 -> 147 ms, 5 M x 4-D float k = 128 103 -> 49 ms, 60 k x 12-D k = 15 125 ->
-// 2.6 ms, 1 M x 3-D k = 32 8.6 -> 5.0 ms.  Queries per warp: 2 and 4 share the
-// leaves' loads and box reads equally well (4 runs at 16 warps per SM: 49-51
-// and 146 ms), 8 spill (61 and 333 ms).  Blocks of 8 warps on consecutive tiles
-// share the L1 better than blocks of 4 (6-D: 146 against 154 ms).
+// not memory (L2 hits 98 %): 5 550 warp instructions per query of a 1 M-point
+// 6-D double join at 0.52 per cycle and scheduler; 65 leaves per query at 10 M.
+// Search kernels of whole joins, one warp per query on the grid's ring
+// (k_search.cu) before, this now: 10 M x 6-D double k = 16 790 -> 129 ms, 5 M x
+// 4-D float k = 128 103 -> 45 ms, 60 k x 12-D k = 15 125 -> 2.2 ms, 1 M x 3-D
+// k = 32 9.6 -> 4.2-4.9 ms.  Queries per warp, measured before the points lay in
+// rows per leaf: 2 at 24 warps per SM 147 and 49 ms, 4 at 16 warps 146 and 51
+// ms, 8 spill (333 and 61 ms).  Blocks of 8 warps on consecutive tiles share
+// the L1 better than blocks of 4 (4 queries per warp, 6-D: 146 against 154 ms).
 #pragma once
 
 #include <cmath>
