@@ -92,6 +92,9 @@ constexpr int wave_rows() {
   return (DI > 0 && DI <= 2) ? KNNSJ_WAVE_ROWS_LO : KNNSJ_WAVE_ROWS_HI;
 }
 constexpr int WARP_WORDS = 256 + 2 * MAX_RUNS + 8;  // per-warp u32 scratch: bins, runS, runP
+// Dynamic shared memory of a block; one warp's share stays under 140 KB (a
+// selection buffer of 128 KB, the words below, a query of MAX_D doubles).
+constexpr size_t SEARCH_MAX_SMEM = 200 * 1024;
 constexpr int FILTER_QUEUE = 64;  // double data: candidates that passed the float prefilter
 template <typename T>
 constexpr int warp_words() {
@@ -658,10 +661,10 @@ void launch_one(const SearchParams<T>& prm, int wpb_req, int sm_count, cudaStrea
                           (D == 0 ? (size_t)MAX_D * sizeof(T) : 0);
   int wpb = SEARCH_THREADS / 32;
   if (wpb_req > 0 && wpb_req < wpb) wpb = wpb_req;
-  while (wpb > 1 && per_warp * wpb > 200 * 1024) wpb--;
+  while (wpb > 1 && per_warp * wpb > SEARCH_MAX_SMEM) wpb--;
   const size_t smem = per_warp * wpb;
   auto kern = search_kernel<T, D, DI>;
-  KNNSJ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_dynamic_smem(kern, SEARCH_MAX_SMEM);
   int per_sm = 0;
   KNNSJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, wpb * 32, smem));
   if (per_sm < 1) throw StatusError{KNNSJ_ERR_UNSUPPORTED, "search kernel does not fit"};
@@ -772,9 +775,9 @@ void launch_brute(const SearchLaunch<T>& a, cudaStream_t s) {
   p.rowsum = a.rowsum;
   const size_t per_warp = (size_t)p.B * sizeof(typename Key<T>::type) + 256 * 4;
   int wpb = BRUTE_THREADS / 32;
-  while (wpb > 1 && per_warp * wpb + a.d * sizeof(T) > 200 * 1024) wpb--;
+  while (wpb > 1 && per_warp * wpb + a.d * sizeof(T) > SEARCH_MAX_SMEM) wpb--;
   const size_t smem = per_warp * wpb + a.d * sizeof(T);
-  KNNSJ_CUDA(cudaFuncSetAttribute(brute_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_dynamic_smem(brute_kernel<T>, SEARCH_MAX_SMEM);
   brute_kernel<T><<<a.nq, wpb * 32, smem, s>>>(p);
   KNNSJ_CHECK_LAUNCH();
 }

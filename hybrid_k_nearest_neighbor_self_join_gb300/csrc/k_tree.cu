@@ -399,7 +399,7 @@ void launch_tree_build(const T* xs, const T* minmax, uint64_t n, uint32_t d, Tre
   }
   const uint32_t rd = std::min<uint32_t>(d, REFINE_DIMS);
   const size_t smem = (size_t)rd * BLOCK_PTS * 4;
-  KNNSJ_CUDA(cudaFuncSetAttribute(tree_refine_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_dynamic_smem(tree_refine_kernel<T>, (size_t)REFINE_DIMS * BLOCK_PTS * 4);
   tree_refine_kernel<T><<<(unsigned)((n + BLOCK_PTS - 1) / BLOCK_PTS), REFINE_THREADS, smem, s>>>(
       xs, n, d, rd, sc.sort.vals[cur], const_cast<T*>(t.ps), const_cast<float*>(t.psf), const_cast<uint32_t*>(t.id),
       const_cast<float*>(t.box), t.dims, t.count[0], t.levels > 1 ? t.offset[1] : 0xffffffffu);

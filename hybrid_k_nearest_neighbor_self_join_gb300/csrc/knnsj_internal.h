@@ -43,6 +43,16 @@ extern thread_local bool g_forbid_alloc;
     ++::knnsj::g_launches;                   \
   } while (0)
 
+// Lets `kern` be launched with up to `limit` bytes of dynamic shared memory.
+// The limit belongs to the kernel, not to the launch, and batched joins launch
+// the same kernel from several host threads with different sizes: `limit` is
+// the most any launch of the kernel asks for, so that no thread lowers it
+// between another's setting and its launch (which the runtime then refuses).
+template <typename F>
+inline void allow_dynamic_smem(F* kern, size_t limit) {
+  KNNSJ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+}
+
 // ---- device buffers of one join (cached across calls, grow-only) --------
 // A fixed device region carved out by bump allocation (no cudaMalloc).
 struct Arena {

@@ -47,6 +47,7 @@ constexpr int TREE_THREADS = 256;  // largest block
 constexpr int tree_min_blocks(int d) { return d == 3 ? 4 : 3; }
 constexpr int TREE_Q = 2;          // queries per warp
 constexpr int TREE_QUEUE = 64;     // double data: candidates that passed the float screen, per query
+constexpr size_t TREE_MAX_SMEM = 110 * 1024;  // dynamic shared memory of a block
 constexpr int TREE_STACK = 6;      // levels above the leaves' parents
 constexpr uint32_t TREE_CHUNK = 64;  // tiles of a block's run of consecutive queries
 
@@ -548,10 +549,10 @@ void launch_tree_one(const TreeParams<T>& p, int sm_count, cudaStream_t s) {
                           (sizeof(T) == 8 ? (size_t)Q * TREE_QUEUE * 4 + (size_t)Q * p.d * sizeof(T) : 0) +
                           (D == 0 ? (size_t)Q * p.d * 4 : 0);
   int wpb = TREE_THREADS / 32;
-  while (wpb > 1 && per_warp * wpb > 110 * 1024) wpb--;
-  const size_t smem = per_warp * wpb;
+  while (wpb > 1 && per_warp * wpb > TREE_MAX_SMEM) wpb--;
+  const size_t smem = per_warp * wpb;  // (one warp: 16 KB at most)
   auto kern = tree_kernel<T, D, Q>;
-  KNNSJ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_dynamic_smem(kern, TREE_MAX_SMEM);
   int per_sm = 0;
   KNNSJ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, wpb * 32, smem));
   if (per_sm < 1) throw StatusError{KNNSJ_ERR_UNSUPPORTED, "tree search kernel does not fit"};
