@@ -77,12 +77,13 @@ struct TreeParams {
 // float chain) whose square is at most the result, and so has the gap to any
 // box that holds it: rounding moves a coordinate x by at most 2^-24 |x|, the
 // point lies within |q| + sqrt(t) of the origin, and the chain of d terms is
-// off by a few ulps.
+// off by (d + 8) 2^-23 of the result and, where terms are subnormal, by half of
+// the smallest float (2^-149) per term.
 __device__ __forceinline__ float screen_bound(float t_up, float qnorm, uint32_t d) {
   const float s = __fsqrt_ru(__fmul_ru(t_up, 1.0f + 1.0f / 1048576.0f));
   const float e = __fmaf_ru(__fmaf_ru(2.0f, qnorm, s), 1.01f / 16777216.0f, 1e-37f);
   const float w = __fadd_ru(s, e);
-  return __fmul_ru(__fmul_ru(w, w), 1.0f + (float)(d + 8) * 1.2e-7f);
+  return __fadd_ru(__fmul_ru(__fmul_ru(w, w), 1.0f + (float)(d + 8) * 1.2e-7f), __uint_as_float(d));  // (d 2^-149)
 }
 
 // A warp's state in shared memory, one entry per query of its tile.  The scan
