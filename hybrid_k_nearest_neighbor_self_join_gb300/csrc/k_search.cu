@@ -499,7 +499,9 @@ __global__ void __launch_bounds__(SEARCH_THREADS, search_min_blocks<T, D, DI>())
             auto filt_thr = [&]() -> float {
               const double t = (double)Kt::acc(st.tau);
               const double sq = sqrt(t * (1.0 + 1.0 / 1099511627776.0)) + (double)p.filt_e1;
-              return __double2float_ru((1.0 + (double)(p.d + 4) * 1.1920928955078125e-07) * sq * sq);
+              // (d 2^-149: terms that are subnormal in float round by half of that each)
+              return __double2float_ru((1.0 + (double)(p.d + 4) * 1.1920928955078125e-07) * sq * sq +
+                                       (double)p.d * 1.401298464324817e-45);
             };
             float tf = filt_thr();
             uint32_t qn = 0;

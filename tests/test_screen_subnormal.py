@@ -38,14 +38,11 @@ def check(x, k, queries, di=0):
 
 # offsets whose squares round up in float (in 12, 16 and 40 equal terms the chain
 # ends above a bound without the absolute term)
-TREES = ["1"]
 SIZES = [2.7e-23, 1.7e-22, 4.5e-22, 1.2e-21, 3.6e-21]
 
 
-@pytest.mark.parametrize("tree", TREES)
 @pytest.mark.parametrize("d", [12, 16, 40])
-def test_corners(monkeypatch, tree, d):
-    monkeypatch.setenv("KNNSJ_TREE", tree)
+def test_corners(d):
     rng = np.random.default_rng(d)
     for c in SIZES:
         x = c * rng.choice([-1.0, 1.0], (3000, d))
@@ -54,11 +51,9 @@ def test_corners(monkeypatch, tree, d):
         check(x, 40, centre)
 
 
-@pytest.mark.parametrize("tree", TREES)
 @pytest.mark.parametrize("d", [12, 40, 128])
 @pytest.mark.parametrize("beside", [False, True])
-def test_cloud(monkeypatch, tree, d, beside):
-    monkeypatch.setenv("KNNSJ_TREE", tree)
+def test_cloud(d, beside):
     rng = np.random.default_rng(100 + d)
     for c in SIZES:
         x = rng.uniform(-c, c, (1500, d))
@@ -66,3 +61,15 @@ def test_cloud(monkeypatch, tree, d, beside):
             x = np.concatenate([x, rng.uniform(0.5, 1.0, (1500, d))])
         # (more indexed dimensions are refused beside points near 1: over 2^64 cells)
         check(x, 24, np.arange(0, 1500, 7), di=2)
+
+
+@pytest.mark.parametrize("d", [12, 40])
+def test_corners_ring_search(monkeypatch, d):
+    # the grid's ring search has a screen of its own
+    monkeypatch.setenv("KNNSJ_TREE", "0")
+    rng = np.random.default_rng(200 + d)
+    for c in SIZES[1:4]:
+        x = c * rng.choice([-1.0, 1.0], (700, d))
+        centre = rng.integers(0, 700, 8)
+        x[centre] = 0.0
+        check(x, 20, centre)
