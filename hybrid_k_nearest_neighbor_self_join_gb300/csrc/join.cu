@@ -338,7 +338,7 @@ struct SmallHead {
   unsigned long long cand;
   double avg[2];
   unsigned long long defer_total;       // all queries handed over by the tile search in this join
-  unsigned long long tree_rmax;         // tree search: largest radius grown or searched (bits)
+  unsigned long long tree_rmax;         // tree search: largest radius searched (bits)
   uint32_t tree_fail[2];                // tree search: failures of its first two passes
   uint32_t mlp_err;                     // the tensor-core radius MLP timed out
   uint32_t pad;
@@ -1462,7 +1462,7 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
     kernel_ms += elapsed(4, 5);
     alg_bytes += (double)iter * n * d * sizeof(T) + (double)queries_run * d * sizeof(T) +
                  (double)n * K * (4.0 + sizeof(T));
-    rmax_seen = std::max(qrad ? rmax_seen : (double)r, decode_radius<T>(head.tree_rmax));
+    rmax_seen = decode_radius<T>(head.tree_rmax);
   }
   if (mlp_err && cfg.verbose)  // rows are still exact: the affected queries started at eps0
     fprintf(stderr, "knnsj: the tensor-core radius model timed out (%u); those queries started at eps0\n", mlp_err);

@@ -351,7 +351,7 @@ struct TreeLaunch {
   uint32_t* fail_mask = nullptr;     // bits of the failed queries (cleared before the pass)
   uint32_t* fail_count = nullptr;
   T* grow = nullptr;                 // grown radii of the failures, by original id
-  unsigned long long* rmax_bits = nullptr;  // largest radius grown or (without radii) searched
+  unsigned long long* rmax_bits = nullptr;  // largest radius searched or grown
   unsigned long long* cand_count = nullptr;
 };
 template <typename T>

@@ -68,7 +68,7 @@ struct TreeParams {
   uint32_t* fail_mask;     // bits of the failed queries (cleared before the pass)
   uint32_t* fail_count;
   T* grow;                 // radii of the failed queries by original id
-  unsigned long long* rmax_bits;  // largest radius grown or (without radii) searched
+  unsigned long long* rmax_bits;  // largest radius searched or grown
   unsigned long long* cand_count;
 };
 
@@ -463,7 +463,12 @@ __global__ void __launch_bounds__(TREE_THREADS, tree_min_blocks(D)) tree_kernel(
     if (first >= have) continue;
     // (one lane per query: the threshold of a double radius takes square roots)
     const uint32_t my_pos = own * 32 + nth_bit(leaf_mask, min(first + min(lane, Q - 1), have - 1));
-    const T thr = p.unbounded ? (T)INFINITY : within_threshold(p.qradius ? p.qradius[p.t.id[my_pos]] : p.radius);
+    T thr = (T)INFINITY;
+    if (!p.unbounded) {
+      const T r0 = p.qradius ? p.qradius[p.t.id[my_pos]] : p.radius;
+      thr = within_threshold(r0);
+      rmax = r0 > rmax ? r0 : rmax;
+    }
 #pragma unroll
     for (int i = 0; i < Q; i++) {
       const uint32_t at_pos = __shfl_sync(FULL, my_pos, i);
@@ -535,6 +540,11 @@ __global__ void __launch_bounds__(TREE_THREADS, tree_min_blocks(D)) tree_kernel(
       }
       __syncwarp();
     }
+  }
+#pragma unroll
+  for (int i = 1; i < Q; i++) {  // (the lanes that read the queries' radii)
+    const T o = __shfl_sync(FULL, rmax, i);
+    rmax = o > rmax ? o : rmax;
   }
   if (lane == 0) {
     if (t.scanned) atomicAdd(p.cand_count, 32ull * t.scanned);
