@@ -1042,11 +1042,12 @@ static bool run_graph_passes(Workspace& w, SearchLaunch<T> a, LoopCtl& c, LoopCt
 
 // Builds the tree over the grid's point buffers (the grid is not searched
 // afterwards) and runs the passes: each reads its query count on the device,
-// so nothing waits for the host in between.
+// so nothing waits for the host in between (verbose 2: a line per pass, each
+// waited for).
 template <typename T>
-static void run_tree(Workspace& w, const Prepared<T>& P, uint64_t n, uint32_t d,
-                     uint32_t di, uint32_t K, T* qrad, int32_t* d_ids, T* d_dists, double* rowsum, uint32_t* list, SmallDev* sm,
-                           cudaStream_t s) {
+static void run_tree(Workspace& w, const Prepared<T>& P, uint64_t n, uint32_t d, uint32_t di, uint32_t K, T* qrad,
+                     int32_t* d_ids, T* d_dists, double* rowsum, uint32_t* list, SmallDev* sm, int verbose,
+                     cudaStream_t s) {
   BoxTree<T> t;
   tree_shape(n, d, t.count, t.offset, &t.levels, &t.nodes);
   t.dims = std::min(d, TREE_DIMS);
@@ -1083,19 +1084,38 @@ static void run_tree(Workspace& w, const Prepared<T>& P, uint64_t n, uint32_t d,
   a.grow = (T*)w.qradius.get(n * sizeof(T));
   a.rmax_bits = &sm->tree_rmax;
   a.cand_count = &sm->cand;
+  const bool report = verbose >= 2;
+  uint32_t nq = (uint32_t)n;
+  auto pass = [&](int i) {
+    const bool timed = report && w.ev[6] && w.ev[7];
+    if (timed) KNNSJ_CUDA(cudaEventRecord(w.ev[6], s));
+    launch_tree_search<T>(a, w.sm_count, s);
+    if (timed) KNNSJ_CUDA(cudaEventRecord(w.ev[7], s));
+    if (!report) return;
+    SmallHead head;
+    read_small(w, &head, static_cast<SmallHead*>(sm), sizeof(head), s);
+    const uint32_t nfail = i < 2 ? head.tree_fail[i] : 0u;
+    float ms = 0.f;
+    if (timed) KNNSJ_CUDA(cudaEventElapsedTime(&ms, w.ev[6], w.ev[7]));
+    if (nq > 0)
+      fprintf(stderr, "knnsj: pass %d: %u queries, %u failed, box tree, %s (largest so far %g), %.3f ms, "
+              "candidates so far %llu\n", i, nq, nfail, a.unbounded ? "no radius" : "radii", decode_radius<T>(head.tree_rmax),
+              ms, head.cand);
+    nq = nfail;
+  };
   if (w.ev[4]) KNNSJ_CUDA(cudaEventRecord(w.ev[4], s));
-  launch_tree_search<T>(a, w.sm_count, s);
+  pass(0);
   a.qmask = mask[0];
   a.nq_dev = &sm->tree_fail[0];
   a.qradius = a.grow;
   a.fail_mask = mask[1];
   a.fail_count = &sm->tree_fail[1];
-  launch_tree_search<T>(a, w.sm_count, s);
+  pass(1);
   a.qmask = mask[1];
   a.nq_dev = &sm->tree_fail[1];
   a.qradius = nullptr;
   a.unbounded = 1;
-  launch_tree_search<T>(a, w.sm_count, s);
+  pass(2);
   if (w.ev[5]) KNNSJ_CUDA(cudaEventRecord(w.ev[5], s));
 }
 
@@ -1317,7 +1337,7 @@ void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_ao
   // 6b. the box tree: every query at its starting radius, the failures at a
   // radius grown from what they found, and the rest without a radius
   if (use_tree) {
-    run_tree<T>(w, P, n, d, di, K, qrad, d_ids, d_dists, rowsum, list[0], sm, s);
+    run_tree<T>(w, P, n, d, di, K, qrad, d_ids, d_dists, rowsum, list[0], sm, cfg.verbose, s);
     regrids = 1;  // the index was rebuilt once, as the tree
     nq = 0;       // (the passes are counted from the head below)
   }
