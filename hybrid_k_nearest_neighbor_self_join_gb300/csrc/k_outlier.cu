@@ -41,8 +41,7 @@ __global__ void in_degree_kernel(const int32_t* __restrict__ ids, uint64_t count
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
        i += (uint64_t)gridDim.x * blockDim.x) {
     const int32_t id = ids[i];
-    // (a degree is at most n < 2^31: its low word is counted)
-    if (id >= 0 && (uint64_t)id < n) atomicAdd(reinterpret_cast<uint32_t*>(&indeg[id]), 1u);
+    if (id >= 0 && (uint64_t)id < n) atomicAdd(&indeg[id], 1ull);
   }
 }
 
