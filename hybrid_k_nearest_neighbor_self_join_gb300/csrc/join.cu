@@ -141,11 +141,23 @@ void Workspace::pinned_release() {
   h_pinned_bytes = 0;
 }
 
+// Page-locked, mapped host memory, or false where there is none to be had.
+// KNNSJ_TEST_PINNED_KB=n (tests only): blocks above n KB are refused.
+static bool alloc_pinned(void** p, size_t bytes) {
+  const char* e = std::getenv("KNNSJ_TEST_PINNED_KB");
+  if (!(e && bytes > (size_t)std::atoll(e) * 1024) &&
+      cudaHostAlloc(p, bytes, cudaHostAllocMapped) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
 void* Workspace::pinned(size_t need) {
   if (need > h_pinned_bytes) {
     if (g_forbid_alloc) throw StatusError{KNNSJ_ERR_EXCEEDS_FIXED_SCRATCH, "pinned buffer in a fixed-scratch join"};
     pinned_release();
-    KNNSJ_CUDA(cudaMallocHost(&h_pinned, need));
+    if (!alloc_pinned(&h_pinned, need)) return nullptr;
     h_pinned_bytes = need;
   }
   return h_pinned;
@@ -163,13 +175,15 @@ void Workspace::ensure_copy_stream() {
   if (!copy_stream) KNNSJ_CUDA(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
   for (auto& e : chunk_ev)
     if (!e) KNNSJ_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  ensure_mail();
+  if (!ensure_mail()) throw CudaError{cudaErrorMemoryAllocation, "mailbox of streamed rows"};
 }
 
-void Workspace::ensure_mail() {
-  if (mail_host || g_forbid_alloc) return;  // (fixed-scratch joins copy into pageable memory)
-  KNNSJ_CUDA(cudaHostAlloc(&mail_host, MAIL_BYTES, cudaHostAllocMapped));
+bool Workspace::ensure_mail() {
+  if (mail_host) return true;
+  // (joins with fixed scratch, or without page-locked memory, copy into pageable memory)
+  if (g_forbid_alloc || !alloc_pinned(&mail_host, MAIL_BYTES)) return false;
   KNNSJ_CUDA(cudaHostGetDevicePointer(&mail_dev, mail_host, 0));
+  return true;
 }
 
 bool Workspace::ensure_stage(int blocks) {
@@ -178,11 +192,7 @@ bool Workspace::ensure_stage(int blocks) {
     if (stage) cudaFreeHost(stage);
     stage = nullptr;
     stage_blocks = 0;
-    if (cudaMallocHost(&stage, (size_t)blocks * STAGE_BYTES) != cudaSuccess) {
-      cudaGetLastError();
-      stage = nullptr;
-      return false;
-    }
+    if (!alloc_pinned(&stage, (size_t)blocks * STAGE_BYTES)) return false;
     stage_blocks = blocks;
   }
   for (int i = 0; i < blocks; i++)
@@ -284,8 +294,7 @@ __global__ void __launch_bounds__(1024) collect_kernel(uint32_t* __restrict__ ds
 static void read_pieces(Workspace& w, std::initializer_list<Piece> pieces, cudaStream_t s) {
   size_t bytes = 0;
   for (const Piece& p : pieces) bytes += p.bytes;
-  w.ensure_mail();
-  if (w.mail_host && bytes <= MAIL_BYTES / 2 && pieces.size() <= MAX_PIECES) {
+  if (w.ensure_mail() && bytes <= MAIL_BYTES / 2 && pieces.size() <= MAX_PIECES) {
     PieceList l{};
     int i = 0;
     for (const Piece& p : pieces) {
@@ -808,13 +817,19 @@ static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T
       sp = sample.data();
     } else if (!g_forbid_alloc) {
       // gathered by a kernel straight into mapped memory (a strided copy of
-      // rows of a few bytes is slow on the copy engines)
-      T* host = (T*)w.pinned(ns * d * sizeof(T));
-      void* dev = nullptr;
-      KNNSJ_CUDA(cudaHostGetDevicePointer(&dev, host, 0));
+      // rows of a few bytes is slow on the copy engines); without page-locked
+      // memory through the buffer of the columns, which are not there yet
+      const size_t bytes = ns * d * sizeof(T);
+      T* host = (T*)w.pinned(bytes);
+      void* dev = w.xs.get(n * d * sizeof(T));
+      if (host) KNNSJ_CUDA(cudaHostGetDevicePointer(&dev, host, 0));
       launch_gather_rows<T>(d_aos, ns, 100, d, (T*)dev, s);
+      if (!host) {
+        sample.resize(ns * d);
+        KNNSJ_CUDA(cudaMemcpyAsync(sample.data(), dev, bytes, cudaMemcpyDeviceToHost, s));
+      }
       KNNSJ_CUDA(cudaStreamSynchronize(s));
-      sp = host;
+      sp = host ? host : sample.data();
     } else {
       sample.resize(ns * d);
       KNNSJ_CUDA(cudaMemcpy2DAsync(sample.data(), d * sizeof(T), d_aos, 100 * d * sizeof(T),

@@ -393,9 +393,9 @@ struct Workspace {
   size_t h_pinned_bytes = 0;
   void ensure_stream();
   void ensure_copy_stream();
-  void ensure_mail();
+  bool ensure_mail();          // false: no pinned memory to be had
   bool ensure_stage(int blocks);  // false: no pinned memory to be had
-  void* pinned(size_t need);
+  void* pinned(size_t need);   // nullptr: no pinned memory to be had
   void pinned_release();
   void release_all();
   void attach_arena(Arena* a);  // every buffer carves from `a` from now on
