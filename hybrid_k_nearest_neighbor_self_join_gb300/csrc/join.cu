@@ -142,12 +142,13 @@ void Workspace::pinned_release() {
 }
 
 // Page-locked, mapped host memory, or false where there is none to be had.
-// KNNSJ_TEST_PINNED_KB=n (tests only): blocks above n KB are refused.
+// KNNSJ_TEST_PINNED_KB=n (tests only): blocks above n KB are refused, with a line
+// on stderr.
 static bool alloc_pinned(void** p, size_t bytes) {
   const char* e = std::getenv("KNNSJ_TEST_PINNED_KB");
-  if (!(e && bytes > (size_t)std::atoll(e) * 1024) &&
-      cudaHostAlloc(p, bytes, cudaHostAllocMapped) == cudaSuccess)
-    return true;
+  const bool refuse = e && bytes > (size_t)std::atoll(e) * 1024;
+  if (!refuse && cudaHostAlloc(p, bytes, cudaHostAllocMapped) == cudaSuccess) return true;
+  if (refuse) fprintf(stderr, "knnsj: refused %zu bytes of page-locked memory\n", bytes);
   cudaGetLastError();
   *p = nullptr;
   return false;
@@ -817,10 +818,11 @@ static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T
       sp = sample.data();
     } else if (!g_forbid_alloc) {
       // gathered by a kernel straight into mapped memory (a strided copy of
-      // rows of a few bytes is slow on the copy engines); without page-locked
-      // memory through the buffer of the columns, which are not there yet
+      // rows of a few bytes is slow on the copy engines); large samples, and any
+      // where there is no page-locked memory, through the buffer of the columns,
+      // which are not there yet
       const size_t bytes = ns * d * sizeof(T);
-      T* host = (T*)w.pinned(bytes);
+      T* host = bytes <= SAMPLE_PINNED_BYTES ? (T*)w.pinned(bytes) : nullptr;
       void* dev = w.xs.get(n * d * sizeof(T));
       if (host) KNNSJ_CUDA(cudaHostGetDevicePointer(&dev, host, 0));
       launch_gather_rows<T>(d_aos, ns, 100, d, (T*)dev, s);

@@ -59,3 +59,26 @@ def test_same_rows(tmp_path, kb):
     assert sorted(want) == sorted(got)
     for name in want:
         assert want[name].tobytes() == got[name].tobytes(), name
+
+
+def test_largest_block():
+    # the blocks a workspace keeps are at most 16 MB, whatever the size of the
+    # data: here the dimension sample alone has 32 MB
+    body = """
+import numpy as np, torch
+import hybrid_k_nearest_neighbor_self_join_gb300 as kj
+n = 200_000_000
+g = torch.Generator(device="cuda"); g.manual_seed(1)
+x = torch.rand(n, 2, generator=g, device="cuda", dtype=torch.float64)
+x[:, 1] *= 1.5
+ids = torch.empty(n, 2, dtype=torch.int32, device="cuda")
+dists = torch.empty(n, 2, dtype=x.dtype, device="cuda")
+torch.cuda.synchronize()
+st = kj.selfjoin_device(x.data_ptr(), np.float64, n, 2, 1, ids.data_ptr(), dists.data_ptr())
+print("perm", *st["perm"][:2])
+"""
+    env = dict(os.environ, PYTHONPATH=ROOT, KNNSJ_TEST_PINNED_KB="16384")
+    p = subprocess.run([sys.executable, "-c", body], env=env, cwd=ROOT, timeout=300, capture_output=True, text=True)
+    assert p.returncode == 0, p.stderr[-2000:]
+    assert "perm 1 0" in p.stdout  # the sample's order: larger variance first
+    assert "refused" not in p.stderr
