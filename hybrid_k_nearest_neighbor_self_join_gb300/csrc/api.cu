@@ -439,11 +439,13 @@ void device_join(const T* data, uint64_t n, uint32_t d, uint32_t k, const JoinCo
 struct ShapeKey {
   int dtype;
   uint32_t d, di, K;
+  bool tree;  // searched through the box tree, which takes no shape
   bool operator<(const ShapeKey& o) const {
     if (dtype != o.dtype) return dtype < o.dtype;
     if (d != o.d) return d < o.d;
     if (di != o.di) return di < o.di;
-    return K < o.K;
+    if (K != o.K) return K < o.K;
+    return tree < o.tree;
   }
 };
 
@@ -470,8 +472,9 @@ std::vector<SearchShape> candidate_shapes(uint32_t K) {
 
 // Tuned shapes persist across processes in a text file named by
 // KNNSJ_TUNE_CACHE: one line per class, "<device> dtype d di K warps qchunk
-// buffer" (the device's name with blanks replaced by '_'); lines of other
-// devices are kept as they are.  The file is read the first time the batched
+// buffer" (the device's name with blanks replaced by '_'), with the word "tree"
+// behind it for a class searched through the box tree, which has no shape (0 0
+// 0); lines of other devices are kept as they are.  The file is read the first time the batched
 // join runs on a device, and rewritten (through a temporary file and a
 // rename) whenever classes were tuned.  Only shapes the tuner itself would
 // try are taken from it.
@@ -504,15 +507,18 @@ void load_tune_cache(int dev) {
   FILE* f = std::fopen(path, "r");
   if (!f) return;
   const std::string tag = device_tag(dev);
-  char name[256];
+  char line[512], name[256], path_word[16];
   int dt = 0;
   unsigned d = 0, di = 0, K = 0;
   SearchShape sh;
-  while (std::fscanf(f, "%255s %d %u %u %u %d %d %d", name, &dt, &d, &di, &K, &sh.warps_per_block, &sh.qchunk,
-                     &sh.buffer) == 8) {
-    if (tag == name && tunable_shape(K, sh)) {
-      g_tuned[ShapeKey{dt, d, di, K}] = sh;
-      g_measured.insert(ShapeKey{dt, d, di, K});
+  while (std::fgets(line, sizeof(line), f)) {
+    const int fields = std::sscanf(line, "%255s %d %u %u %u %d %d %d %15s", name, &dt, &d, &di, &K, &sh.warps_per_block,
+                                   &sh.qchunk, &sh.buffer, path_word);
+    const bool tree = fields == 9 && std::strcmp(path_word, "tree") == 0;
+    if ((fields == 8 || tree) && tag == name && tunable_shape(K, sh)) {
+      const ShapeKey key{dt, d, di, K, tree};
+      g_tuned[key] = sh;
+      g_measured.insert(key);
     }
   }
   std::fclose(f);
@@ -537,8 +543,8 @@ void save_tune_cache(int dev) {
   std::fputs(keep.c_str(), f);
   for (const auto& kv : g_tuned)
     if (g_measured.count(kv.first))
-      std::fprintf(f, "%s %d %u %u %u %d %d %d\n", tag.c_str(), kv.first.dtype, kv.first.d, kv.first.di, kv.first.K,
-                 kv.second.warps_per_block, kv.second.qchunk, kv.second.buffer);
+      std::fprintf(f, "%s %d %u %u %u %d %d %d%s\n", tag.c_str(), kv.first.dtype, kv.first.d, kv.first.di, kv.first.K,
+                   kv.second.warps_per_block, kv.second.qchunk, kv.second.buffer, kv.first.tree ? " tree" : "");
   const bool ok = std::fclose(f) == 0;
   if (ok) std::rename(tmp.c_str(), path);
   else std::remove(tmp.c_str());
@@ -574,7 +580,11 @@ void run_batched(knnsj_set* sets, const std::vector<uint32_t>& order, const std:
   }
   const int code = sizeof(T) == 4 ? KNNSJ_F32 : KNNSJ_F64;
   auto key_of = [&](uint32_t i) {
-    return ShapeKey{code, sets[i].d, cfgs[i].num_indexed_dims, sets[i].k + 1};
+    const JoinConfig& c = cfgs[i];
+    const knnsj_set& t = sets[i];
+    const bool streams = c.direct_rows == 0 && c.row_chunks >= 2 && t.n >= ROW_STREAM_MIN_ROWS &&
+                         mapped_host_pointer(t.out_ids) && mapped_host_pointer(t.out_dists);
+    return ShapeKey{code, t.d, c.num_indexed_dims, t.k + 1, join_takes_tree(c, t.n, t.d, t.k + 1, sizeof(T), streams)};
   };
   auto join_one = [&](Workspace& w, uint32_t i, const SearchShape& sh, knnsj_stats* st) {
     JoinConfig c = cfgs[i];
@@ -584,7 +594,9 @@ void run_batched(knnsj_set* sets, const std::vector<uint32_t>& order, const std:
     host_join_ws<T>(w, (const T*)sets[i].data, sets[i].n, sets[i].d, sets[i].k, c, sets[i].out_ids,
                     (T*)sets[i].out_dists, st, false, STAGE_THREADS_BATCHED);
   };
-  // autotune the classes seen for the first time, on their largest set
+  // autotune the classes seen for the first time, on their largest set: the
+  // shapes are those of the ring search, so sets that go through the box tree
+  // are classes of their own and are not joined to try any
   load_tune_cache(dev);
   bool tuned_now = false;
   const char* at = env("KNNSJ_AUTOTUNE");
@@ -598,7 +610,11 @@ void run_batched(knnsj_set* sets, const std::vector<uint32_t>& order, const std:
   for (const auto& kv : largest) {
     if (g_tuned.count(kv.first)) continue;
     SearchShape best;
-    if (tune && sets[kv.second].n >= 20000) {
+    const bool record = tune && sets[kv.second].n >= 20000;
+    if (record && kv.first.tree) {  // nothing to try
+      g_measured.insert(kv.first);
+      tuned_now = true;
+    } else if (record) {
       Workspace& w = *pool.ws[0];
       knnsj_stats st;
       std::memset(&st, 0, sizeof(st));

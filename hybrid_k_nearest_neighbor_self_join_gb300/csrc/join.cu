@@ -797,6 +797,11 @@ static bool tree_applies(const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t
   return n >= TREE_LEARNED_2D_MIN && !(cfg.tile_search && tile_search_applies(d, di, K, 1, sizeof(T)));
 }
 
+bool join_takes_tree(const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t K, size_t elem, bool streams) {
+  return elem == 4 ? tree_applies<float>(cfg, n, d, cfg.num_indexed_dims, K, 0.0, streams)
+                   : tree_applies<double>(cfg, n, d, cfg.num_indexed_dims, K, 0.0, streams);
+}
+
 template <typename T>
 static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_aos, uint64_t n, uint32_t d,
                     uint32_t k, knnsj_stats* st, cudaStream_t s, Prepared<T>* P, bool will_stream = false,

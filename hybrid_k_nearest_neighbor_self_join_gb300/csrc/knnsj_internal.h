@@ -416,6 +416,10 @@ template <typename T>
 void run_join(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T* h_aos, uint64_t n, uint32_t d,
               uint32_t k, int32_t* d_ids, T* d_dists, knnsj_stats* st, cudaStream_t s,
               RowStream* rows = nullptr, double* rowsum = nullptr);
+// Whether such a join is searched through the box tree, as far as that is known
+// without the data: double coordinates too large for the float screen take the
+// ring search all the same.
+bool join_takes_tree(const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t K, size_t elem, bool streams);
 template <typename T>
 void finish_row_stream(Workspace& w, const RowStream& rows, const int32_t* d_ids, const T* d_dists, uint32_t K,
                        cudaStream_t s);
