@@ -15,13 +15,12 @@
 #include <mutex>
 #include <set>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #ifdef KNNSJ_BUILD_DTYPE_DOUBLE
 #define KNNSJ_KNNJOINPY_DOUBLE 1
 #endif
+#include "host_threads.h"
 #include "knnsj_host.h"
 #include "knnsj_internal.h"
 
@@ -281,14 +280,7 @@ bool copy_out_staged(Workspace& w, const CopyOut (&seg)[2], int threads, cudaStr
     }
     if (e != cudaSuccess) failed.store(e);
   };
-  std::vector<std::thread> pool;
-  try {
-    for (int t = 1; t < threads; t++) pool.emplace_back(work, t);
-  } catch (const std::system_error&) {
-    // fewer threads share the blocks
-  }
-  work(0);
-  for (std::thread& t : pool) t.join();
+  run_on_threads(threads, work);
   if (failed.load() != cudaSuccess) throw CudaError{(cudaError_t)failed.load(), "copy of the result table"};
   return true;
 }
@@ -656,10 +648,7 @@ void run_batched(knnsj_set* sets, const std::vector<uint32_t>& order, const std:
       sets[i].status = guarded([&] { join_one(w, i, sh, &st); }, nullptr);
     }
   };
-  std::vector<std::thread> th;
-  for (int wi = 1; wi < nw; wi++) th.emplace_back(worker, wi);
-  worker(0);
-  for (auto& t : th) t.join();
+  run_on_threads(nw, worker);
   for (const knnsj_stats& st : per) {
     agg->iterations += st.iterations;
     agg->regrids += st.regrids;
