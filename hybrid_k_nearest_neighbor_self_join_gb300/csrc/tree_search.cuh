@@ -553,15 +553,23 @@ __global__ void __launch_bounds__(TREE_THREADS, tree_min_blocks(D)) tree_kernel(
   }
 }
 
+// Dynamic shared memory of one warp: a selection buffer of B keys per query, the
+// shared state, the reduction's bins, the walk's stack; double data also the
+// queue and the queries, a runtime dimension count the queries in float.
+template <typename T, int D, int Q>
+constexpr size_t tree_warp_bytes(uint32_t B, uint32_t d) {
+  return (size_t)Q * B * sizeof(typename Key<T>::type) + sizeof(TreeState<T, Q>) + 1024 + TREE_STACK * 128 +
+         (sizeof(T) == 8 ? (size_t)Q * TREE_QUEUE * 4 + (size_t)Q * d * sizeof(T) : 0) +
+         (D == 0 ? (size_t)Q * d * 4 : 0);
+}
+static_assert(tree_warp_bytes<double, 0, TREE_Q>(HIST_MAX_B, MAX_D) <= TREE_MAX_SMEM, "one warp fits a block");
+
 template <typename T, int D, int Q>
 void launch_tree_one(const TreeParams<T>& p, int sm_count, cudaStream_t s) {
-  const size_t per_warp = (size_t)Q * p.B * sizeof(typename Key<T>::type) + sizeof(TreeState<T, Q>) + 1024 +
-                          TREE_STACK * 128 +
-                          (sizeof(T) == 8 ? (size_t)Q * TREE_QUEUE * 4 + (size_t)Q * p.d * sizeof(T) : 0) +
-                          (D == 0 ? (size_t)Q * p.d * 4 : 0);
+  const size_t per_warp = tree_warp_bytes<T, D, Q>(p.B, p.d);
   int wpb = TREE_THREADS / 32;
   while (wpb > 1 && per_warp * wpb > TREE_MAX_SMEM) wpb--;
-  const size_t smem = per_warp * wpb;  // (one warp: 16 KB at most)
+  const size_t smem = per_warp * wpb;
   auto kern = tree_kernel<T, D, Q>;
   allow_dynamic_smem(kern, TREE_MAX_SMEM);
   int per_sm = 0;
