@@ -773,7 +773,8 @@ struct Prepared {
 // 120, float and double, BETA 0.025 (ring over tree time):
 //   four and more dimensions: the ring of cells visits several times the
 //     points and most first passes fail; 1.4x (4-D) to 27x (12-D);
-//   three dimensions: 0.98-3.1x, the tile kernel's learned joins included;
+//   three dimensions: 0.98-3.1x, the tile kernel's learned joins of up to a
+//     million points included;
 //   two dimensions, a uniform radius: 0.97-2.5x from 30 000 points on (most
 //     first passes fail; the tree needs no schedule of passes), 1.0-1.3x at
 //     2 000 (0.8x at k = 120, where few passes fail);
@@ -785,6 +786,19 @@ struct Prepared {
 //     points, k = 200: 1.06-5.7x float, 0.88-4.6x double, k = 223 double
 //     0.7-2.1x, k = 1000 0.65-1.0x, k = 4000 0.5-0.7x.
 constexpr uint64_t TREE_LEARNED_2D_MIN = 1000000;
+
+// Large three-dimensional learned joins whose occupied cells hold about k + 1
+// points each (an evenly filled space or surface, with a dense cell table) stay
+// with the query tiles: their rings are a few cells wide and nearly every query
+// succeeds at once.  Uneven density makes wide rings beside dense cells and
+// outliers.  Whole joins, k = 1 to 64, tree time over tile time:
+//   0.8 (k + 1) points per occupied cell or more (uniform, a sphere's surface):
+//     0.8-1.1x at 300 000 points, 0.99-1.4x at 1 M, 1.06-1.5x at 5 M, 1.2-1.7x at
+//     20 M;
+//   fewer, 1 to 20 M: normal data (0.3-0.8 of k + 1) 0.4-1.5x with no order in n
+//     or k (the tiles wait for a few outliers), mixtures 0.1-1.1x.
+constexpr uint64_t TILE_3D_MIN = 1000000;
+constexpr double TILE_3D_FILL = 0.8;
 template <typename T>
 static bool tree_applies(const JoinConfig& cfg, uint64_t n, uint32_t d, uint32_t di, uint32_t K, double max_abs,
                          bool will_stream) {
@@ -920,6 +934,17 @@ static void prepare(Workspace& w, const JoinConfig& cfg, const T* d_aos, const T
   // its cells are only counted, where a bitmap of them fits (up to 32 MB, or
   // what the fixed scratch array grants a dense table).
   if (use_tree) *use_tree = tree_applies<T>(cfg, n, d, di, k + 1, max_abs, will_stream);
+  if (use_tree && *use_tree && cfg.tree_search == 1 && d == 3 && n >= TILE_3D_MIN &&
+      cfg.radius_mode == KNNSJ_RADIUS_LEARNED && query_tiles<T>(cfg, d, di, k + 1)) {
+    const GridGeom<T> g = grid_geometry<T>(di, P->mn, P->mx, eps0);
+    if (dense_table(cfg, n, g.total_cells)) {
+      launch_count_cells<T>(xs, n, g, (uint32_t*)w.dstart.get((size_t)((g.total_cells + 31) / 32) * 4), &sm->C0, s);
+      unsigned long long occupied = 0;
+      read_small(w, &occupied, &sm->C0, sizeof(occupied), s);
+      launch_zero_words(&sm->C0, sizeof(sm->C0), s);  // (counted again by the grid)
+      *use_tree = (double)n < TILE_3D_FILL * (double)(k + 1) * (double)occupied;
+    }
+  }
   if (use_tree && *use_tree && cfg.radius_mode != KNNSJ_RADIUS_LEARNED) {
     const GridGeom<T> g = grid_geometry<T>(di, P->mn, P->mx, eps0);
     P->grid.geom = g;

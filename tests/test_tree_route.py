@@ -102,3 +102,21 @@ def test_fixed_scratch(monkeypatch, capfd, d, dtype, mode):
     torch.cuda.synchronize()
     assert "box tree" in capfd.readouterr().err
     check_brute(x, ids.cpu().numpy(), dists.cpu().numpy(), np.arange(0, n, 2_311))
+
+
+def test_large_learned_3d_by_density(monkeypatch, capfd):
+    # evenly filled space stays with the query tiles from a million points on,
+    # uneven density goes through the tree; fewer points always
+    rng = np.random.default_rng(7)
+    monkeypatch.setenv("KNNSJ_VERBOSE", "2")
+    for x, tree in ((rng.random((1_000_000, 3)), False), (datasets.gmm(1_000_000, 3, 12, 0.2, 8), True),
+                    (rng.random((999_999, 3)), True)):
+        x = x.astype(F)
+        capfd.readouterr()
+        ids, dists, st = kj.selfjoin(x, 8, radius_mode=LEARNED, return_stats=True)
+        assert ("box tree" in capfd.readouterr().err) == tree
+        check_brute(x, ids, dists, np.arange(0, len(x), 20_011))
+        perm = st["perm"][:3]
+        lo, width = x[:, perm].min(0), F(st["eps0"])
+        cells = np.unique(((x[:, perm] - lo) / width).astype(np.int64) @ np.array([1, 1 << 20, 1 << 40]))
+        assert abs(st["nonempty_cells"] - len(cells)) <= len(cells) * 1e-3
