@@ -191,7 +191,8 @@ constexpr float LEARNED_LOG_MARGIN = 0.08f;
 
 // Largest ring half-width (in cells of the eps0 grid) a learned radius may
 // start with: keeps a ring at most ~1024 rows; growth beyond is handled by
-// the retry schedule and grid rebuilds.
+// the retry schedule and grid rebuilds.  (Ring and tile searches; a join through
+// the box tree has no rings and takes 64 at every dimension count.)
 double learned_max_cells(uint32_t di) {
   if (const char* e = std::getenv("KNNSJ_LEARNED_MAX_CELLS")) {  // tuning override
     const double v = std::atof(e);

@@ -1,7 +1,7 @@
 // k_tile.cu -- range search of low-dimensional float data by tiles of
-// queries: one warp owns QPT queries (4 by default) that are neighbours in
-// Morton order of their cells, 32 / QPT lanes per query, and the tile's
-// queries share one pass over the candidates of the union of their rings.
+// queries: one warp owns QPT queries (4 by default) that are neighbours along
+// a space-filling curve of their cells (Hilbert in two dimensions, Morton in
+// three), 32 / QPT lanes per query, and the tile's queries share one pass over the candidates of the union of their rings.
 //
 // Replaces, for the first search pass of float data with two or three
 // dimensions (all indexed) and k+1 <= 65, the same reference steps as
@@ -23,7 +23,7 @@
 //   3. the single pass over the candidates: every key (squared distance,
 //      id) within the query's radius goes to the query's list in shared
 //      memory, its slot from a ballot over the query's lanes (no atomics);
-//      a query that finds more keys than the list holds (0.2 % of the sky
+//      a query that finds more keys than the list holds (0.04 % of the sky
 //      join) is handed to search_kernel, one that finds fewer than K fails
 //      (the reference's acceptance rule, GPU.cu:3659-3669);
 //   4. each accepted query's list is sorted by the whole warp as 32-bit words
