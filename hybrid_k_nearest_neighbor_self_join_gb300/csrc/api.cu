@@ -20,6 +20,7 @@
 #ifdef KNNSJ_BUILD_DTYPE_DOUBLE
 #define KNNSJ_KNNJOINPY_DOUBLE 1
 #endif
+#include "host_pages.h"
 #include "host_threads.h"
 #include "knnsj_host.h"
 #include "knnsj_internal.h"
@@ -237,23 +238,39 @@ struct SyncOnExit {
 // for 68 MB; eight threads fault the pages in and fill them in 1.4 ms, 0.4 ms
 // of copies behind them.  (Faulting the pages in ahead, while the join runs,
 // makes the runtime's copy slower, not faster: 25 ms.)
+//
+// Into pages that are in memory the runtime copies at the link's rate, the
+// staged copy at 70 GB/s: whole joins with their table in a reused array,
+// runtime and staged, 8 MB 0.72 and 1.1 ms, 64 MB 1.3 and 2.2, 128 MB 1.8 and
+// 3.1.  Above that the runtime's copy takes several times as long now and then
+// (256 MB in ten arrays in turn 3-31 ms, on average 3.1 to 20 per round, staged
+// 5.5; 512 MB 7.7-25 and 12.5).  With part of the pages absent the two meet at
+// about three eighths of them (64 MB) or a quarter (790 MB).
 struct CopyOut {
   void* dst;
   const void* src;
   size_t bytes;
 };
 constexpr size_t STAGED_MIN_BYTES = 4u << 20;  // smaller tables: threads cost more than they save
+constexpr size_t WARM_MAX_BYTES = 128u << 20;  // larger ones are staged also into pages in memory
 constexpr int STAGE_THREADS_BATCHED = 2;       // beside each of the batched joins' workers
 
-// False: not ordinary pageable memory, too small, or no staging memory.
+// False: not ordinary pageable memory, too small, in memory already (joins by
+// themselves: with several workers the runtime's copies slow one another down,
+// 30 sets into arrays from recycled memory 71-134 ms against 40), or no staging
+// memory.
 bool copy_out_staged(Workspace& w, const CopyOut (&seg)[2], int threads, cudaStream_t s) {
-  if (seg[0].bytes + seg[1].bytes < STAGED_MIN_BYTES) return false;
+  const size_t bytes = seg[0].bytes + seg[1].bytes;
+  if (bytes < STAGED_MIN_BYTES) return false;
   for (const CopyOut& c : seg) {
     cudaPointerAttributes a{};
     const cudaError_t e = cudaPointerGetAttributes(&a, c.dst);
     cudaGetLastError();
     if (e == cudaSuccess && a.type != cudaMemoryTypeUnregistered) return false;
   }
+  if (threads > STAGE_THREADS_BATCHED && bytes <= WARM_MAX_BYTES &&
+      (absent_bytes(seg[0].dst, seg[0].bytes) + absent_bytes(seg[1].dst, seg[1].bytes)) * 4 <= bytes)
+    return false;
   threads = std::min(threads, STAGE_BLOCKS);
   if (!w.ensure_stage(threads)) return false;
   int dev = 0;
